@@ -2031,6 +2031,21 @@ static void zcol_work_split(TmaGeom &g, long long ncols, int D, long long grid)
     }
 }
 
+// Stages of a ring that `niss` issuers share, stage j issued by issuer j mod
+// niss, with nb accumulator regions: at most `fit`.  An issuer waits for a
+// slot's full barrier by parity, so it must know that the slot's previous
+// load (stage j - S) has landed: before that, the parity of stage j already
+// reads as complete, and the issuer would run on a slab still in flight and
+// arrive twice on barriers counted for one.  It knows when that stage was its
+// own (S a multiple of niss), or when a region it has waited for was last used
+// by that stage or a later one (its stage j - niss waited for the drains of
+// stage j - niss - nb, which follow every earlier stage's MMAs: S >= niss + nb).
+// Otherwise two loads that land out of order are enough to break the ring.
+static int ring_stages(int fit, int niss, int nb)
+{
+    return fit >= niss + nb ? fit : fit - fit % niss;
+}
+
 // the concatenated-dz z-column convolution (conv_zcat_kernel) when its
 // weights stay resident and 4+ stages fit; false leaves the layer to the
 // others.  IAC_DENOISE_ZCAT=0 in the environment turns it off (for comparing
@@ -2072,7 +2087,7 @@ static bool launch_zcat(const ConvArgs &a, const TmaGeom &g0, uint32_t budget, c
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
-        int per_sm = 0, S = 0;
+        int per_sm = 0, S = 0, niss = Z::NISS;
         for (int want = Z::PER_SM; want >= 1 && per_sm == 0; want--) {
             const uint32_t share = std::min(budget, (228u * 1024u) / (uint32_t)want - 2048u);
             if (share <= g.wres_bytes) continue;
@@ -2095,17 +2110,21 @@ static bool launch_zcat(const ConvArgs &a, const TmaGeom &g0, uint32_t budget, c
             }
         }
         if (per_sm == 0) return false;
+        if (S == 3) niss = 3;  // all three stages in use, one issuer each
+        S = ring_stages(S, niss, Z::NB);
+        if (S < 2) return false;
         g.S = S;
         const long long grid_max = ((long long)per_sm * std::max(1, a.sms) + NG - 1) / NG;  // per channel group
         const long long grid0 = std::min<long long>(nb * g.T * a.D, grid_max);
         zcol_work_split(g, nb * g.T, a.D, grid0);
         const long long grid = g.ZC ? std::min<long long>(grid0, g.nitems) : grid0;
         const uint32_t smem = g.wres_bytes + (uint32_t)S * g.stage_bytes;
-        auto k = conv_zcat_kernel<CIN, COUT, Z::COUTH, Z::NB, Z::NISS, Z::PER_SM>;
+        auto k = niss == 3 ? conv_zcat_kernel<CIN, COUT, Z::COUTH, Z::NB, 3, Z::PER_SM>
+                           : conv_zcat_kernel<CIN, COUT, Z::COUTH, Z::NB, Z::NISS, Z::PER_SM>;
         err = smem_attributes(k, smem);
         if (err != cudaSuccess) return true;
         ++launch_count;
-        k<<<dim3((unsigned)grid, NG), 32 * (ZCAT_ISSUER0 + Z::NISS), smem, s>>>(map, a, g);
+        k<<<dim3((unsigned)grid, NG), 32 * (ZCAT_ISSUER0 + niss), smem, s>>>(map, a, g);
         err = cudaGetLastError();
         return true;
     }
@@ -2145,7 +2164,7 @@ static bool launch_zpair(const ConvArgs &a, cudaStream_t s, cudaError_t &err)
         g.wstage_bytes = 0;
         const uint32_t budget = 227u * 1024u - 2048u;
         if (g.wres_bytes + 4u * g.stage_bytes > budget) return false;
-        g.S = (int)std::min<uint32_t>(8u, (budget - g.wres_bytes) / g.stage_bytes);
+        g.S = ring_stages((int)std::min<uint32_t>(8u, (budget - g.wres_bytes) / g.stage_bytes), ZPAIR_NISS, ZPAIR_NB);
         constexpr int NG = COUT / 16;  // output-channel groups (blockIdx.y)
         const long long grid_max = ((long long)std::max(1, a.sms) + NG - 1) / NG;  // one CTA per SM
         const long long grid0 = std::min<long long>(nb * g.T * a.D, grid_max);
