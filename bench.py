@@ -320,11 +320,11 @@ def measured_bf16_tflops():
 
 def pair_box_radius(C, ctas_per_sm):
     """Half-width of the pair kernel's shared-memory box around q = 0 for a
-    tuning row (the library's rule: 10, shrunk until ctas_per_sm boxes of
-    (R + 1)(2R + 1)^2 words fit in 200 KB, at most the mesh centre)."""
-    budget = (200 << 10) // max(1, ctas_per_sm)
-    r = min(10, C)
-    while r > 0 and 8 * (r + 1) * (2 * r + 1) ** 2 > budget:
+    large batch (the library's rule: 22, shrunk until the boxes of an SM's CTAs
+    of (R + 1)(2R + 1)^2 32-bit words fit in 184 KB, at most the mesh centre)."""
+    budget = (184 << 10) // max(1, ctas_per_sm)
+    r = min(22, C)
+    while r > 0 and 4 * (r + 1) * (2 * r + 1) ** 2 > budget:
         r -= 1
     return r
 
@@ -462,7 +462,8 @@ def run_ours(args):
     updates = pairs - int(len(ph_h))
     upd_rate = updates / (ms_kernel * 1e-3)
     tun = ctx.sparse_tuning(S)
-    R = pair_box_radius((S - 1) // 2, tun["ctas_per_sm"])
+    # the threads of a setting run in as few CTAs of up to 1 024 as hold them
+    R = pair_box_radius((S - 1) // 2, -(-tun["block_threads"] * tun["ctas_per_sm"] // 1024))
     self_sum = 1000.0 * float((ph_h[:, 3].astype(np.float64) ** 2).sum())
     share = box_value_share(half, S, R, self_sum) if R > 0 else 0.0
 
@@ -545,17 +546,15 @@ def run_ours(args):
                             "accumulate into a device-resident mesh that is folded and read back once at "
                             "the end of the run; d2h per step = the 65 MB mesh / steps"},
             "e2e_sync_call": sync_call,
-            "roofline": {"bound": "l2_atomic", "achieved": upd_rate, "peak": atomic_peak,
-                         "unit": "updates/s", "frac": upd_rate / atomic_peak, "traffic": None,
+            "roofline": {"bound": "l2_atomic", "achieved": upd_rate * (1 - share), "peak": atomic_peak,
+                         "unit": "updates/s", "frac": upd_rate * (1 - share) / atomic_peak, "traffic": None,
                          "peak_source": "measured in this run: 2^30 scattered u64 atomic adds into a buffer "
                                         "of the half mesh's size (iac_bench_scatter_add)",
                          "kernel": "sparse_pairs_kernel (+ planner)", "kernel_ms": ms_kernel,
                          "updates_per_launch": updates,
-                         "box": {"radius": R, "value_share": share,
-                                 "l2_updates_per_s": upd_rate * (1 - share),
-                                 "l2_frac": upd_rate * (1 - share) / atomic_peak,
+                         "box": {"radius": R, "value_share": share, "updates_per_s_with_the_box": upd_rate,
                                  "note": "updates within R of q = 0 go to a per-CTA shared-memory box; "
-                                         "l2_frac counts only the updates that reach L2 (box share "
+                                         "achieved counts only the updates that reach L2 (box share "
                                          "estimated from the mesh value it holds)"},
                          "atomic_peak_u32_per_s": atomic_peak_u32,
                          "traffic_note": "DRAM bytes are not measured in the run; the half mesh stays in "

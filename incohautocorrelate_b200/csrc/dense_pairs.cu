@@ -401,36 +401,6 @@ __device__ __forceinline__ void cq_pairs_win(const DenseArgs &a, const Window &w
 }
 
 // ---- two consecutive staged pixels per step, FP32 work as f32x2 pairs ----
-// add/sub/mul.rn.f32x2 (sm_100) round each lane exactly as the scalar
-// instruction does, so the pair of results is bit-identical to two scalar ops.
-// Unlike scalar mul.rn/add.rn, a packed multiply whose product feeds a packed
-// add can come out of ptxas as one fused FFMA2 (one rounding instead of two),
-// so products are only packed where no add consumes them.
-__device__ __forceinline__ float2 f2sub(float2 a, float2 b)
-{
-    float2 r;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "sub.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 f2add(float2 a, float2 b)
-{
-    float2 r;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 f2mul(float2 a, float2 b)
-{
-    float2 r;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "mul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-
 // round half away from zero of both lanes, as ints (see round_half_away)
 __device__ __forceinline__ int2 f2round_half_away(float2 x)
 {

@@ -6,29 +6,26 @@
 // many frames.
 //
 // Work decomposition.  A frame of n photons has n(n-1)/2 distinct pairs plus
-// n self pairs.  The planner (one CTA) gives every frame
-// max(1, ceil(pairs / tile_pairs)) tiles and writes the exclusive prefix sum of
-// those counts: the device work queue.  The pair kernel is persistent: each
-// CTA pops the next tile index with one atomic, finds its frame by binary
-// search over the prefix table and walks the tile's pairs, one pair per thread
-// per step.  Frames of 5 or 2 500 photons therefore cost in proportion to their
-// pair count, and no CTA waits on another.
-//
-// Pair enumeration.  Local pair l of a frame maps to
-//   d = l / n + 1,  i = l % n,  j = (i + d) mod n
-// which lists every unordered pair {i, j}, i != j, exactly once for l in
-// [0, n(n-1)/2) (a circulant walk: offsets d = 1 .. floor((n-1)/2) for every
-// i, plus d = n/2 for i < n/2 when n is even).  Consecutive threads take
-// consecutive i at the same offset d, so their photon loads are contiguous.
-// The pair is then evaluated exactly as the reference's work item does for
-// ind = min(i, j) and i = max(i, j): q = k_lo - k_hi.
+// n self pairs.  Every unordered pair {i, j}, i != j, is (i, i + d mod n) for
+// exactly one offset d = 1 .. floor(n/2) (d = n/2 only for i < n/2 when n is
+// even).  The offsets are cut into chunks of L steps; an item is (photon i,
+// chunk), a unit 32 consecutive items: a warp whose lanes hold one photon each
+// and walk the L partners i + d, so the partner loads of a step are 512
+// contiguous bytes and a step needs one load, no division and no ordering of
+// its two photons.  Frames are laid end to end by cost (units x (L + overhead))
+// and every warp of the launch takes an equal contiguous share of the batch's
+// cost: no work queue, no barrier between frames.  L comes from the batch's
+// pair count, so that a single event still spreads over the GPU.
 //
 // Exactness.  All float operations are the reference's, in its order, as
-// explicitly rounded intrinsics (no contraction into FMA); sqrt is IEEE; the
-// value (double)v_lo * v_hi * Multiplicator is truncated to uint64 as the C
-// cast does.  Self pairs add (uint64)(v*v*Mult) at q = 0, which the reference
-// writes to half-mesh voxel (C, C, 0) without a mirror for every second-level
-// interpolation mode; they are summed per tile and added with one atomic.
+// explicitly rounded intrinsics (no contraction into FMA); the value
+// (double)v_lo * v_hi * Multiplicator is truncated to uint64 as the C cast
+// does.  Swapping a pair's photons negates q exactly, and nearest binning of
+// -q is the point reflection of that of q, which the half mesh folds back; the
+// linear modes restore the reference's order q = k_lo - k_hi.  Self pairs add
+// (uint64)(v*v*Mult) at q = 0, which the reference writes to half-mesh voxel
+// (C, C, 0) without a mirror for every second-level interpolation mode; they
+// are summed per warp and added with one atomic.
 //
 // The half mesh accumulates with 64-bit atomic adds in L2 (the 201^3 half mesh
 // is 32.6 MB and stays L2-resident).  Writes whose voxel would fall outside the
@@ -39,35 +36,13 @@
 #include <cstring>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "iac_internal.cuh"
 
 namespace iac {
 
-struct SparseArgs {
-    const float4 *__restrict__ photons;
-    const uint64_t *__restrict__ offsets;
-    const float *__restrict__ rot;
-    const unsigned long long *__restrict__ tile_off;  // nframes + 1
-    unsigned long long *__restrict__ half;
-    unsigned long long *queue;
-    DeviceCounters *counters;
-    uint32_t nframes;
-    uint32_t tile_pairs;
-    int S, C, half_ss;
-    uint32_t plane;  // S * S (the half mesh has fewer than 2^32 words for S <= 1621)
-    float maxq;
-    float maxq2;  // largest float s with sqrtf(s) <= maxq: |q| > maxq  <=>  |q|^2 > maxq2
-    float vpdq;   // (float)Voxel_per_dq
-    double mult;
-    float mult_f;                           // Multiplicator as float when it is an integer <= 1024
-    const unsigned char *__restrict__ small_counts;  // per frame: counts are integers in [0, 128]
-    int cache_hints;  // 1: mesh atomics evict-last, photon loads evict-first in L2
-    uint64_t mesh_policy;  // set inside the kernel when cache_hints is on
-    int box_r;        // half-width of the shared-memory box around q = 0 (0: none)
-    int box_w;        // 2 * box_r + 1
-    uint32_t box_base;  // shared-memory address of the box's low words (set inside the kernel)
-    uint32_t box_hi;    // shared-memory address of its high words (set inside the kernel)
-};
+namespace cg = cooperative_groups;
 
 // L2 cache policies (PTX createpolicy) for the pair kernel: the half mesh is
 // kept resident while the photon stream passes through.
@@ -81,6 +56,12 @@ __device__ __forceinline__ uint64_t l2_policy_evict_first()
 {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t l2_policy_normal()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_unchanged.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
 __device__ __forceinline__ void red_add_hint(unsigned long long *addr, unsigned long long v, uint64_t pol)
@@ -97,151 +78,428 @@ __device__ __forceinline__ float4 ld_photon_hint(const float4 *p, uint64_t pol)
 }
 
 // ---------------------------------------------------------------------------
-// planner: tiles per frame, exclusive scan, queue reset (one CTA)
+// the walk over a batch's pairs
+// ---------------------------------------------------------------------------
+constexpr uint32_t PAIR_STEPS_MAX = 32;   // steps of a unit (partners a lane walks) at most
+constexpr uint32_t PAIR_UNIT_COST = 3;    // a unit's set-up in units of a step, for the shares
+constexpr uint32_t PAIR_DIRECT = 256;     // frames a CTA plans by itself, without the planner's launch
+
+// what the planner leaves for the walking kernels, before the table of frame starts
+struct PlanHeader {
+    unsigned long long cost;   // of the whole batch
+    unsigned long long pairs;  // distinct pairs of the whole batch
+    uint32_t steps;            // the batch's step limit
+    uint32_t next;             // chunks of the batch taken so far
+};
+
+struct WalkArgs {
+    const float4 *__restrict__ photons;
+    const uint64_t *__restrict__ offsets;
+    PlanHeader *head;                                   // written by the planner; null: planned by the CTA
+    const unsigned long long *__restrict__ cost_off;    // nframes + 1
+    uint32_t nframes;
+    uint32_t steps_max;
+};
+
+__device__ __forceinline__ unsigned long long frame_pairs(uint32_t n)
+{
+    return n ? (unsigned long long)n * (n - 1) / 2 : 0ull;
+}
+
+// chunks and steps of a frame of n photons under the batch's step limit
+struct FrameShape {
+    uint32_t nc, L;
+    unsigned long long units;
+};
+__device__ __forceinline__ FrameShape frame_shape(uint32_t n, uint32_t steps)
+{
+    // steps run two at a time, so L is even; of the two smallest chunk counts the
+    // one with the less padding and set-up
+    const uint32_t half = n >> 1;
+    const uint32_t nc0 = max(1u, (half + steps - 1) / steps), nc1 = nc0 + 1;
+    const uint32_t L0 = ((half + nc0 - 1) / nc0 + 1) & ~1u, L1 = ((half + nc1 - 1) / nc1 + 1) & ~1u;
+    FrameShape s;
+    const bool more = nc1 * (L1 + PAIR_UNIT_COST) < nc0 * (L0 + PAIR_UNIT_COST);
+    s.nc = more ? nc1 : nc0;
+    s.L = more ? L1 : L0;
+    s.units = ((unsigned long long)n * s.nc + 31) / 32;
+    return s;
+}
+__device__ __forceinline__ unsigned long long frame_cost(uint32_t n, uint32_t steps)
+{
+    const FrameShape s = frame_shape(n, steps);
+    return s.units * (s.L + PAIR_UNIT_COST);
+}
+// the step limit that leaves every warp of the launch about two units or more
+__device__ __forceinline__ uint32_t batch_steps(unsigned long long pairs, uint32_t warps, uint32_t steps_max)
+{
+    const unsigned long long s = pairs / (64ull * warps);
+    return (uint32_t)max(1ull, min((unsigned long long)steps_max, s));
+}
+
+// ---------------------------------------------------------------------------
+// planner: the exclusive prefix sum of the frames' costs (the first cluster),
+// and per frame a flag for the pair kernel's fast path (the other CTAs, one warp
+// per frame): the largest photon count if all photon values are integers in
+// [1, 128], so that v_lo * v_hi * Mult (Mult an integer <= 1024) is at most 2^24
+// and exact in FP32, FLAG_VALUES for other values, and 0 (no fast path) unless
+// the k-vectors are finite and the rows of the rotation are short enough
+// (row_limit2, a little over 1 for the mesh of a detector) that no pair within
+// MaxQ can leave the mesh.
+// Bound by reading the photons once: 61 us for 100 000 frames of 11 M photons
+// (one CTA walking 98 frames per thread took 146 us, the check another 36).
 // ---------------------------------------------------------------------------
 constexpr int PLAN_THREADS = 1024;
+constexpr int PLAN_CTAS = 8;  // CTAs of the scanning cluster (the portable cluster size)
 
-__device__ __forceinline__ unsigned long long frame_tiles(const uint64_t *off, uint32_t f,
-                                                          uint32_t tile_pairs)
+__device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v, unsigned long long *warp_sums)
 {
-    const unsigned long long n = off[f + 1] - off[f];
-    if (n == 0) return 0;
-    const unsigned long long pairs = n * (n - 1) / 2;
-    const unsigned long long t = (pairs + tile_pairs - 1) / tile_pairs;
-    return t > 0 ? t : 1;
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();  // warp_sums may still be read
+    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = v;
+    __syncthreads();
+    unsigned long long t = 0;
+    for (uint32_t w = 0; w < blockDim.x / 32; w++) t += warp_sums[w];
+    return t;
 }
 
-__global__ void __launch_bounds__(PLAN_THREADS)
-    sparse_plan_kernel(const uint64_t *__restrict__ off, uint32_t nframes, uint32_t tile_pairs,
-                       unsigned long long *__restrict__ tile_off, unsigned long long *queue)
+constexpr uint32_t FLAG_VALUES = 129, FLAG_GENERAL = 255;  // 255 is stored as 0
+// the photon's count, or what rules counts or the fast path out
+__device__ __forceinline__ uint32_t fast_count(const float4 p)
+{
+    const bool count = p.w >= 1.0f && p.w <= 128.0f && p.w == truncf(p.w);
+    const bool finite = fabsf(p.x) < INFINITY && fabsf(p.y) < INFINITY && fabsf(p.z) < INFINITY;
+    return !finite ? FLAG_GENERAL : count ? (uint32_t)p.w : FLAG_VALUES;
+}
+__device__ __forceinline__ bool fast_row(const float *r, float row_limit2)
+{
+    return r[0] * r[0] + r[1] * r[1] + r[2] * r[2] <= row_limit2;  // false for a NaN
+}
+
+__global__ void __cluster_dims__(PLAN_CTAS, 1, 1) __launch_bounds__(PLAN_THREADS)
+    sparse_plan_kernel(const uint64_t *__restrict__ off, uint32_t nframes, uint32_t steps_max, uint32_t warps,
+                       unsigned long long *__restrict__ cost_off, PlanHeader *head, const float4 *__restrict__ ph,
+                       const float *__restrict__ rot, float row_limit2, unsigned char *__restrict__ flags)
 {
     __shared__ unsigned long long warp_sums[PLAN_THREADS / 32];
+    __shared__ unsigned long long s_mine[2];  // this CTA's pairs and cost, read by the cluster
     const uint32_t tid = threadIdx.x;
-    const uint32_t chunk = (nframes + PLAN_THREADS - 1) / PLAN_THREADS;
-    const uint32_t f0 = min(nframes, tid * chunk), f1 = min(nframes, f0 + chunk);
-    unsigned long long local = 0;
-    for (uint32_t f = f0; f < f1; f++) local += frame_tiles(off, f, tile_pairs);
-    // block-wide exclusive scan of the per-thread sums
     const int lane = tid & 31, w = tid >> 5;
-    unsigned long long incl = local;
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_sums[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-        unsigned long long v = warp_sums[lane];
-        unsigned long long s = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long u = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += u;
+    if (blockIdx.x >= PLAN_CTAS) {
+        const uint32_t warp = (blockIdx.x - PLAN_CTAS) * (PLAN_THREADS / 32) + w;
+        const uint32_t stride = (gridDim.x - PLAN_CTAS) * (PLAN_THREADS / 32);
+        for (uint32_t f = warp; f < nframes; f += stride) {
+            uint32_t m = lane >= 3 || fast_row(rot + 9 * (size_t)f + 3 * lane, row_limit2) ? 1u : FLAG_GENERAL;
+            const uint64_t end = off[f + 1];
+            for (uint64_t i = off[f] + lane; i < end; i += 128) {  // four loads in flight
+                const float4 p0 = ph[i], p1 = ph[min(i + 32, end - 1)], p2 = ph[min(i + 64, end - 1)],
+                             p3 = ph[min(i + 96, end - 1)];
+                m = max(max(max(m, fast_count(p0)), max(fast_count(p1), fast_count(p2))), fast_count(p3));
+            }
+            m = __reduce_max_sync(0xffffffffu, m);
+            if (lane == 0) flags[f] = m == FLAG_GENERAL ? 0 : (unsigned char)m;
         }
-        warp_sums[lane] = s - v;  // exclusive warp prefix
+        return;
     }
-    __syncthreads();
-    unsigned long long run = warp_sums[w] + incl - local;
-    for (uint32_t f = f0; f < f1; f++) {
-        tile_off[f] = run;
-        run += frame_tiles(off, f, tile_pairs);
+    cg::cluster_group cl = cg::this_cluster();
+    const uint32_t rank = cl.block_rank();
+    const uint32_t f0 = (uint32_t)((uint64_t)nframes * rank / PLAN_CTAS),
+                   f1 = (uint32_t)((uint64_t)nframes * (rank + 1) / PLAN_CTAS);
+    unsigned long long v = 0;
+    for (uint32_t f = f0 + tid; f < f1; f += PLAN_THREADS) v += frame_pairs((uint32_t)(off[f + 1] - off[f]));
+    v = block_sum_u64(v, warp_sums);
+    if (tid == 0) s_mine[0] = v;
+    cl.sync();
+    unsigned long long pairs = 0;
+    for (int r = 0; r < PLAN_CTAS; r++) pairs += *cl.map_shared_rank(&s_mine[0], r);
+    const uint32_t steps = batch_steps(pairs, warps, steps_max);
+    v = 0;
+    for (uint32_t f = f0 + tid; f < f1; f += PLAN_THREADS) v += frame_cost((uint32_t)(off[f + 1] - off[f]), steps);
+    v = block_sum_u64(v, warp_sums);
+    if (tid == 0) s_mine[1] = v;
+    cl.sync();
+    unsigned long long run = 0, cost = 0;
+    for (uint32_t r = 0; r < PLAN_CTAS; r++) {
+        const unsigned long long c = *cl.map_shared_rank(&s_mine[1], r);
+        run += r < rank ? c : 0ull;
+        cost += c;
     }
-    if (tid == PLAN_THREADS - 1) {
-        tile_off[nframes] = warp_sums[w] + incl;
-        *queue = 0ull;
+    cl.sync();  // no CTA leaves while its sums are read
+    for (uint32_t c0 = f0; c0 < f1; c0 += PLAN_THREADS) {
+        const uint32_t f = c0 + tid;
+        const unsigned long long c = f < f1 ? frame_cost((uint32_t)(off[f + 1] - off[f]), steps) : 0ull;
+        unsigned long long incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        __syncthreads();
+        if (lane == 31) warp_sums[w] = incl;
+        __syncthreads();
+        unsigned long long before = 0, all = 0;
+        for (int k = 0; k < PLAN_THREADS / 32; k++) {
+            const unsigned long long s = warp_sums[k];
+            before += k < w ? s : 0ull;
+            all += s;
+        }
+        if (f < f1) cost_off[f] = run + before + incl - c;
+        run += all;
+    }
+    if (rank == 0 && tid == 0) {
+        cost_off[nframes] = cost;
+        head->cost = cost;
+        head->pairs = pairs;
+        head->steps = steps;
+        head->next = 0u;
     }
 }
 
-// ---------------------------------------------------------------------------
-// per-frame check: are all photon values integers in [0, 128]?  Then the pair
-// value v_lo * v_hi * Mult (Mult an integer <= 1024) is at most 2^24 and the
-// FP32 product is exact, equal to the reference's double product.
-// One warp per frame.
-// ---------------------------------------------------------------------------
-__global__ void sparse_count_check_kernel(const float4 *__restrict__ ph, const uint64_t *__restrict__ off,
-                                          uint32_t nframes, unsigned char *__restrict__ flags)
+// a small batch planned by the CTA itself in shared memory (every thread of
+// the block): s_off gets nframes + 1 starts; returns the header
+__device__ __forceinline__ PlanHeader plan_direct(const WalkArgs &a, uint32_t warps, unsigned long long *s_off,
+                                                  unsigned long long *s_pairs)
 {
-    const uint32_t f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (f >= nframes) return;
-    bool ok = true;
-    for (uint64_t i = off[f] + lane; i < off[f + 1]; i += 32) {
-        const float w = ph[i].w;
-        ok &= (w >= 0.0f) && (w <= 128.0f) && (w == truncf(w));
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) *s_pairs = 0ull;
+    __syncthreads();
+    for (uint32_t f = tid; f < a.nframes; f += blockDim.x) {
+        const uint32_t n = (uint32_t)(a.offsets[f + 1] - a.offsets[f]);
+        s_off[f + 1] = n;
+        if (n > 1) atomicAdd(s_pairs, frame_pairs(n));
     }
-    ok = __all_sync(0xffffffffu, ok);
-    if (lane == 0) flags[f] = ok ? 1 : 0;
+    __syncthreads();
+    PlanHeader h;
+    h.pairs = *s_pairs;
+    h.steps = batch_steps(h.pairs, warps, a.steps_max);
+    h.next = 0u;
+    if (tid < 32) {
+        unsigned long long run = 0;
+        for (uint32_t c0 = 0; c0 < a.nframes; c0 += 32) {
+            const uint32_t f = c0 + tid;
+            unsigned long long incl = f < a.nframes ? frame_cost((uint32_t)s_off[f + 1], h.steps) : 0ull;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long u = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)tid >= o) incl += u;
+            }
+            if (f < a.nframes) s_off[f + 1] = run + incl;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (tid == 0) s_off[0] = 0ull;
+    }
+    __syncthreads();
+    h.cost = s_off[a.nframes];
+    return h;
 }
+
+// last frame f with off[f] <= x, by a whole warp (off[0] <= x < off[nframes])
+__device__ __forceinline__ uint32_t warp_find_frame(const unsigned long long *off, uint32_t nframes,
+                                                    unsigned long long x)
+{
+    uint32_t lo = 0, hi = nframes;  // off[lo] <= x < off[hi]
+    const uint32_t lane = threadIdx.x & 31;
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t at = lo + lane * step;
+        const unsigned below = __ballot_sync(0xffffffffu, at < hi && off[at] <= x);
+        const uint32_t k = 31 - __clz(below);  // lane 0 is always below
+        lo += k * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// The cost [x0, x1) that a CTA's warps take chunks of: the whole batch, from
+// the counter in the header, or for a batch planned in the CTA an equal part of
+// it, from a counter of the CTA.  Shares fixed beforehand left the slowest SM
+// of a 100 000-frame batch 24 % behind the mean.  A CTA takes at most `most`
+// chunks, twice its part of the batch, which bounds what it can add up.
+struct Share {
+    unsigned long long x0, x1;
+    uint32_t chunk;  // cost a warp takes at a time
+    uint32_t most;
+};
+__device__ __forceinline__ Share cta_share(const PlanHeader &h, bool whole)
+{
+    Share s;
+    s.x0 = whole ? 0ull : h.cost * blockIdx.x / gridDim.x;
+    s.x1 = whole ? h.cost : h.cost * (blockIdx.x + 1) / gridDim.x;
+    // about four chunks a warp at least, whole units, and few enough frame searches
+    const unsigned long long part = h.cost / gridDim.x;
+    s.chunk = (uint32_t)max((unsigned long long)(h.steps + PAIR_UNIT_COST), min(128ull, part / (blockDim.x / 8)));
+    s.most = (uint32_t)min(0x7fffffffull, 2 * part / s.chunk + 64);
+    return s;
+}
+
+// The warps of a CTA take chunks of its share in turn (next: its counter; taken:
+// the CTA's own count in shared memory, zero before).  frame(f, base, n) is called (by all lanes) when a warp enters
+// frame f, unit(i, c, active, nc, L) for each unit with the lane's photon i and
+// chunk c (an inactive lane: i = 0).
+template <class Frame, class Unit>
+__device__ __forceinline__ void walk_share(const WalkArgs &a, const PlanHeader &h, const unsigned long long *off,
+                                           const Share &sh, uint32_t *next, uint32_t *taken, Frame frame, Unit unit)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t f = warp_find_frame(off, a.nframes, sh.x0);
+    for (;;) {
+        uint32_t at0 = 0xffffffffu;
+        if (lane == 0 && atomicAdd(taken, 1u) < sh.most) at0 = atomicAdd(next, 1u);
+        at0 = __shfl_sync(0xffffffffu, at0, 0);
+        const unsigned long long start = sh.x0 + (unsigned long long)at0 * sh.chunk;
+        if (at0 == 0xffffffffu || start >= sh.x1) return;
+        const unsigned long long end = min(sh.x1, start + sh.chunk);
+        {   // the frame of `start`, at or after the last one
+            const uint32_t at = f + 1 + lane;
+            const unsigned below = __ballot_sync(0xffffffffu, at <= a.nframes && off[min(at, a.nframes)] <= start);
+            f += __popc(below);
+            if (below == 0xffffffffu) f += warp_find_frame(off + f, a.nframes - f, start);
+        }
+        unsigned long long pos = off[f], skip = start - pos;  // skip: cost of the frame's units before `start`
+        for (uint32_t g = f; pos < end && g < a.nframes; g++) {
+            const uint64_t base = a.offsets[g];
+            const uint32_t n = (uint32_t)(a.offsets[g + 1] - base);
+            const FrameShape s = frame_shape(n, h.steps);
+            const uint32_t cost = s.L + PAIR_UNIT_COST;
+            unsigned long long u = skip ? (skip + cost - 1) / cost : 0ull;  // the units that start in the chunk
+            skip = 0;
+            unsigned long long last = s.units;
+            if (pos + s.units * cost > end) last = (end - pos + cost - 1) / cost;
+            if (u < last) {
+                frame(g, base, n);
+                const unsigned long long items = (unsigned long long)n * s.nc;
+                for (; u < last; u++) {
+                    const unsigned long long t = u * 32 + lane;
+                    const bool active = t < items;
+                    const uint32_t c = !active ? 0u : items < (1ull << 32) ? (uint32_t)t / n : (uint32_t)(t / n);
+                    const uint32_t i = active ? (uint32_t)(t - (unsigned long long)c * n) : 0u;
+                    unit(i, c, active, s.nc, s.L);
+                }
+            }
+            pos += s.units * cost;
+        }
+    }
+}
+
+// the partners of photon i in chunk c: offsets d0 .. d0 + steps - 1
+__device__ __forceinline__ void chunk_steps(uint32_t n, uint32_t i, uint32_t c, uint32_t L, bool active, uint32_t &d0,
+                                            int &steps)
+{
+    const uint32_t half = n >> 1;
+    const uint32_t dmax = (n & 1) ? half : half - (i >= half ? 1u : 0u);
+    d0 = 1 + c * L;
+    steps = active ? (int)min(L, dmax + 1 > d0 ? dmax + 1 - d0 : 0u) : 0;
+}
+
+// Half-width R of the shared-memory box of voxels around q = 0 (ss <= R,
+// |fs - C| <= R, |ms - C| <= R) that each CTA of the pair kernel accumulates
+// privately, by the batch's distinct pairs: none below BOX_PAIRS_SMALL,
+// BOX_R_SMALL below BOX_PAIRS_LARGE, else what the launch has room for.  L2
+// takes scattered adds at about 2e11 per second, one request each, whatever
+// their width, so every add that stays in the box counts: in a 201^3 mesh of
+// the rotated workload R = 22 keeps 32 % of them, R = 10 9 %.  100 000 frames
+// (1.16e9 pairs): 5.01 ms at R = 16, 4.35 at 20, 4.21 at 22 (R = 23 leaves the
+// photons too little L1: 4.18, but a short batch is slower).  The lines between
+// the sizes: 1 000 frames (1.2e7 pairs) 149 us without a box, 139 at R = 10,
+// 148 at 22; 3 000 frames 273, 251 and 229; 300 frames 103, 104 and 118.
+constexpr int BOX_R_MAX = 22;    // 23 x 45 x 45 words: 186 KB
+constexpr int BOX_R_SMALL = 10;
+constexpr unsigned long long BOX_PAIRS_SMALL = 1000000ull, BOX_PAIRS_LARGE = 20000000ull;
+
+struct SparseArgs {
+    WalkArgs walk;
+    const float *__restrict__ rot;
+    unsigned long long *__restrict__ half;
+    DeviceCounters *counters;
+    int S, C, half_ss;
+    uint32_t plane;  // S * S (the half mesh has fewer than 2^32 words for S <= 1621)
+    float maxq2;  // largest float s with sqrtf(s) <= maxq: |q| > maxq  <=>  |q|^2 > maxq2
+    float vpdq;   // (float)Voxel_per_dq
+    float row_limit2;  // squared length of a rotation's rows up to which the fast path applies
+    float neg_zero;  // -0.0f: fma(a, b, -0) is a * b rounded once, and never merges with an add
+    double mult;
+    uint32_t mult_u;                        // Multiplicator when it is an integer <= 1024, else 0
+    const unsigned char *__restrict__ flags;  // per frame: largest count, 0: not the fast path (the planner's check)
+    int check_here;   // no planner ran: the CTA checks its frames itself
+    int fast_ok;      // MaxQ is finite
+    int cache_hints;  // 1: mesh atomics evict-last, photon loads evict-first in L2; else no preference
+    int box_max;      // largest half-width of the shared-memory box that the launch has room for
+    // set inside the kernel
+    uint64_t mesh_policy, photon_policy;
+    float box_lim;    // |rotated component| below this rounds into the box (box_r + 0.5; 0: no box)
+    int center, box_center, box_plane;  // words of the mesh's and the box's centre, words of a box plane
+    int box_r;        // half-width of the box around q = 0 (-1: none)
+    uint32_t box_w;   // 2 * box_r + 1 (0: none)
+    uint32_t box_base;  // shared-memory address of the box
+};
 
 // ---------------------------------------------------------------------------
 // binning helpers (IAC/kernel.cl:349-448)
 // ---------------------------------------------------------------------------
-// v into word k of the shared-memory box, a split 64-bit counter (low words at
-// box_base, high words at box_hi): 32-bit shared atomics are native, 64-bit
-// ones are several times slower, above all where the lanes of a warp meet at
-// one voxel near q = 0
-__device__ __forceinline__ void box_add(const SparseArgs &a, uint32_t k, unsigned long long v)
+__device__ __forceinline__ void mesh_add(const SparseArgs &a, uint32_t word, unsigned long long v)
 {
-    const uint32_t vl = (uint32_t)v;
-    uint32_t old;
-    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a.box_base + 4u * k), "r"(vl) : "memory");
-    const uint32_t up = (uint32_t)(v >> 32) + (old + vl < old ? 1u : 0u);
-    if (up) asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a.box_hi + 4u * k), "r"(up) : "memory");
+    red_add_hint(&a.half[word], v, a.mesh_policy);
 }
 
-__device__ __forceinline__ void hm_put(const SparseArgs &a, int fs, int ms, int ss,
-                                       unsigned long long v)
+__device__ __forceinline__ uint32_t box_add32(const SparseArgs &a, uint32_t k, uint32_t v)
 {
-    if ((unsigned)fs >= (unsigned)a.S || (unsigned)ms >= (unsigned)a.S ||
-        (unsigned)ss >= (unsigned)a.half_ss) {
-        atomicAdd(&a.counters->out_of_mesh, 1ull);
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a.box_base + 4u * k), "r"(v) : "memory");
+    return old;
+}
+
+// 2^32 times `up` at mesh word `word`, or at both words of a mirrored pair of
+// the plane ss = 0
+static __device__ __noinline__ void carry_out(unsigned long long *half, uint32_t word, uint32_t mirror, uint32_t up)
+{
+    atomicAdd(&half[word], (unsigned long long)up << 32);
+    if (mirror != word) atomicAdd(&half[mirror], (unsigned long long)up << 32);
+}
+
+// v at the voxel (r0, r1, r2) relative to the mesh centre, r2 >= 0; a voxel of
+// the plane r2 = 0 and its mirror (-r0, -r1) always receive the same value
+// (q and -q of a pair), so this adds it to both: two adds at the centre itself.
+// The box keeps the low 32 bits of its sums, and one of the two mirrored voxels
+// of its plane 0, which the flush adds to both; what leaves the 32 bits (a
+// carry, seen by the add that caused it, or a value past them) goes straight to
+// the mesh.
+__device__ __forceinline__ void put_pair(const SparseArgs &a, int r0, int r1, int r2, unsigned long long v)
+{
+    const int fs = r0 + a.C, ms = r1 + a.C;
+    const uint32_t word = (uint32_t)fs + (uint32_t)ms * (uint32_t)a.S + (uint32_t)r2 * a.plane;
+    const uint32_t mirror = r2 == 0 ? (uint32_t)(a.C - r0) + (uint32_t)(a.C - r1) * (uint32_t)a.S : word;
+    if ((uint32_t)fs >= (uint32_t)a.S || (uint32_t)ms >= (uint32_t)a.S || r2 >= a.half_ss) {
+        atomicAdd(&a.counters->out_of_mesh, r2 == 0 ? 2ull : 1ull);
         return;
     }
     if (v == 0) return;
-    if (a.box_r) {  // the voxels around q = 0 collect in the CTA's shared-memory box
-        const uint32_t dx = (uint32_t)(fs - a.C + a.box_r), dy = (uint32_t)(ms - a.C + a.box_r);
-        if (dx < (uint32_t)a.box_w && dy < (uint32_t)a.box_w && (uint32_t)ss <= (uint32_t)a.box_r) {
-            const uint32_t k = ((uint32_t)ss * a.box_w + dy) * a.box_w + dx;
-            box_add(a, k, v);
-            return;
-        }
+    if ((uint32_t)(r0 + a.box_r) < a.box_w && (uint32_t)(r1 + a.box_r) < a.box_w && r2 <= a.box_r) {
+        const uint32_t k = ((uint32_t)r2 * a.box_w + (uint32_t)(r1 + a.box_r)) * a.box_w + (uint32_t)(r0 + a.box_r);
+        const uint32_t old = box_add32(a, k, (uint32_t)v);
+        uint32_t up = (uint32_t)(v >> 32) + (old + (uint32_t)v < old ? 1u : 0u);
+        if (r2 == 0 && word == mirror) up *= 2;  // the flush counts the centre twice
+        if (up) carry_out(a.half, word, mirror, up);
+    } else {
+        mesh_add(a, word, v);
+        if (r2 == 0) mesh_add(a, mirror, v);
     }
-    unsigned long long *addr = &a.half[(uint32_t)fs + (uint32_t)ms * (uint32_t)a.S + (uint32_t)ss * a.plane];
-    if (a.cache_hints)
-        red_add_hint(addr, v, a.mesh_policy);
-    else
-        atomicAdd(addr, v);
 }
 
-// AddQToPositiveSS, IAC/kernel.cl:349-372 (q != 0 here; q = 0 is the self pair)
+// AddQToPositiveSS, IAC/kernel.cl:349-372 (q != 0 here; q = 0 is the self
+// pair): ss > 0 as it is, ss < 0 at the point reflection, ss = 0 at both
 __device__ __forceinline__ void add_positive_ss(const SparseArgs &a, int fs, int ms, int ss,
                                                 unsigned long long v)
 {
-    if (ss > 0) {
-        hm_put(a, fs, ms, ss, v);
-    } else {
-        if (ss == 0) hm_put(a, fs, ms, ss, v);
-        hm_put(a, 2 * a.C - fs, 2 * a.C - ms, -ss, v);
-    }
+    const bool neg = ss < 0;
+    put_pair(a, neg ? a.C - fs : fs - a.C, neg ? a.C - ms : ms - a.C, neg ? -ss : ss, v);
 }
 
 // Second-level nearest neighbour of AddRotatedQToMesh (IAC/kernel.cl:380-389)
 // followed by AddQToPositiveSS: fs = C + round(q0), ms = C + round(q1),
-// ss = round(q2); a negative ss goes to the point reflection, ss = 0 goes to
-// both.  (The reference adds the float centre to the rounded float, which is
-// exact for every in-mesh index.)
+// ss = round(q2).  (The reference adds the float centre to the rounded float,
+// which is exact for every in-mesh index.)
 __device__ __forceinline__ void add_nearest(const SparseArgs &a, float q0, float q1, float q2,
                                             unsigned long long v)
 {
-    int fs = a.C + round_away_rz_i(q0);
-    int ms = a.C + round_away_rz_i(q1);
-    int ss = round_away_rz_i(q2);
-    if (ss < 0) {
-        fs = 2 * a.C - fs;
-        ms = 2 * a.C - ms;
-        ss = -ss;
-    }
-    hm_put(a, fs, ms, ss, v);
-    if (ss == 0) hm_put(a, 2 * a.C - fs, 2 * a.C - ms, 0, v);
+    add_positive_ss(a, a.C + round_away_rz_i(q0), a.C + round_away_rz_i(q1), round_away_rz_i(q2), v);
 }
 
 // AddRotatedQToMesh, IAC/kernel.cl:374-448
@@ -275,10 +533,10 @@ __device__ __forceinline__ void add_rotated(const SparseArgs &a, double val, flo
 }
 
 // One distinct pair, the body of the reference's loop for i > ind
-// (IAC/kernel.cl:493-649).
+// (IAC/kernel.cl:493-649): any values, any interpolation.
 template <int DMAP, int I1, int I2>
 __device__ __forceinline__ void bin_pair(const SparseArgs &a, const float4 A, const float4 B,
-                                         const float *R, const bool small_counts)
+                                         const float *R)
 {
     float q0 = fsub(A.x, B.x), q1 = fsub(A.y, B.y), q2 = fsub(A.z, B.z);
     // sqrt(|q|^2) > MaxQ, decided on |q|^2 against the exact float threshold
@@ -290,11 +548,7 @@ __device__ __forceinline__ void bin_pair(const SparseArgs &a, const float4 A, co
     const float Cf = (float)C;
     if (I2 == 0 && (DMAP == 0 || I1 == 0)) {
         // nearest neighbour at the second level: value (ulong)(v_lo * v_hi * Mult)
-        unsigned long long v;
-        if (small_counts)  // integers <= 128 and Mult <= 1024: the float product is exact
-            v = (unsigned long long)__float2uint_rz(fmul(fmul(A.w, B.w), a.mult_f));
-        else
-            v = d2u64(dmul(dmul((double)A.w, (double)B.w), a.mult));
+        const unsigned long long v = d2u64(dmul(dmul((double)A.w, (double)B.w), a.mult));
         float t0 = q0, t1 = q1, t2 = q2;
         if (DMAP) {  // first-level nearest neighbour: back to the voxel centre
             // |q| <= MaxQ * Voxel_per_dq < 2^22 here (MaxQ test, host check)
@@ -345,125 +599,400 @@ __device__ __forceinline__ void bin_pair(const SparseArgs &a, const float4 A, co
 }
 
 // ---------------------------------------------------------------------------
-// persistent pair kernel
+// pair kernel
 // ---------------------------------------------------------------------------
-template <int DMAP, int I1, int I2>
-__global__ void __launch_bounds__(256) sparse_pairs_kernel(SparseArgs a)
+// One rotated pair of the fast path at its nearest voxel (add_nearest, for a q
+// that is finite and inside the mesh): a negative slow component flips the sign
+// of all three first, which is the reflection of a negative ss; the rounding is
+// the sign-magnitude trunc(x + copysign(0.49999997, x)) of round_away_rz_i.
+// What the box holds, and c: SUM_COUNTS sums of c, the product of the counts,
+// which cannot leave 32 bits (the kernel checks the CTA's whole share), so its
+// adds return nothing; SUM_SMALL the values c * Mult, below 2^32, with their
+// carries as in put_pair; SUM_VALUES any values (c is the value).  The adds are
+// predicated rather than branched around: nearly every warp has lanes on either
+// side, and without branches the two pairs of a step overlap.
+enum { SUM_COUNTS, SUM_SMALL, SUM_VALUES };
+template <int SUM>
+__device__ __forceinline__ void put_nearest(const SparseArgs &a, bool on, float x0, float x1, float x2,
+                                            unsigned long long c)
 {
-    uint64_t photon_policy = 0;
-    if (a.cache_hints) {
-        a.mesh_policy = l2_policy_evict_last();
-        photon_policy = l2_policy_evict_first();
+    const bool box = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fabsf(x2)) < a.box_lim;
+    const uint32_t sg = __float_as_uint(x2) & 0x80000000u;
+    x0 = __uint_as_float(__float_as_uint(x0) ^ sg);
+    x1 = __uint_as_float(__float_as_uint(x1) ^ sg);
+    const int r0 = __float2int_rz(fadd(x0, copysignf(0.49999997f, x0)));
+    const int r1 = __float2int_rz(fadd(x1, copysignf(0.49999997f, x1)));
+    const int r2 = __float2int_rz(fadd(fabsf(x2), 0.49999997f));
+    const uint32_t word = (uint32_t)(r0 + r1 * a.S + r2 * (int)a.plane + a.center);
+    const uint32_t bat = a.box_base + 4u * (uint32_t)(r0 + r1 * (int)a.box_w + r2 * a.box_plane + a.box_center);
+    const unsigned long long v = SUM == SUM_VALUES ? c : (unsigned long long)((uint32_t)c * a.mult_u);
+    const int in_box = on && box, in_mesh = on && !box, mirrored = in_mesh && r2 == 0;
+    if (SUM == SUM_COUNTS) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p red.shared.add.u32 [%1], %2;\n\t}" ::"r"(in_box),
+                     "r"(bat), "r"((uint32_t)c)
+                     : "memory");
+    } else if (in_box) {
+        uint32_t old;
+        asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(bat), "r"((uint32_t)v) : "memory");
+        uint32_t up = (uint32_t)(v >> 32) + (old + (uint32_t)v < old ? 1u : 0u);
+        if (up) {
+            if (r2 == 0 && word == (uint32_t)a.center) up *= 2;
+            carry_out(a.half, word, r2 == 0 ? 2u * (uint32_t)a.center - word : word, up);
+        }
     }
-    __shared__ unsigned long long s_tile;
-    __shared__ uint32_t s_frame;
-    __shared__ float s_rot[9];
-    __shared__ int s_small;
-    __shared__ unsigned long long s_self[8];
-    // (box_r + 1) x box_w x box_w split 64-bit counters, [ss][ms][fs]: low words, then high words
-    extern __shared__ uint32_t s_box[];
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p red.global.add.L2::cache_hint.u64 [%1], %2, %3;\n\t}" ::"r"(
+                     in_mesh),
+                 "l"(&a.half[word]), "l"(v), "l"(a.mesh_policy)
+                 : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p red.global.add.L2::cache_hint.u64 [%1], %2, %3;\n\t}" ::"r"(
+                     mirrored),
+                 "l"(&a.half[2u * (uint32_t)a.center - word]), "l"(v), "l"(a.mesh_policy)
+                 : "memory");
+}
 
-    const unsigned long long ntiles = a.tile_off[a.nframes];
+template <int DMAP, int SUM>
+__device__ __forceinline__ void nearest_unit(const SparseArgs &a, const float4 *__restrict__ P, uint32_t n, const float *R,
+                                             uint32_t i, uint32_t d0, int steps)
+{
+    auto load = [&](uint32_t j) { return ld_photon_hint(P + j, a.photon_policy); };
+    const float4 A = load(i);
+    const float2 nz = make_float2(a.neg_zero, a.neg_zero);
+    auto mul = [&](float2 x, float2 y) { return f2fma(x, y, nz); };
+    auto dup = [](float x) { return make_float2(x, x); };
+    uint32_t j = i + d0;
+    if (j >= n) j -= n;
+    auto step = [&](uint32_t x) { return x + 1 == n ? 0u : x + 1; };
+    for (int k = 0; k < steps; k += 2) {
+        const float4 B0 = load(j);
+        j = step(j);
+        const float4 B1 = load(j);
+        j = step(j);
+        float2 q0 = make_float2(fsub(A.x, B0.x), fsub(A.x, B1.x)), q1 = make_float2(fsub(A.y, B0.y), fsub(A.y, B1.y)),
+               q2 = make_float2(fsub(A.z, B0.z), fsub(A.z, B1.z));
+        // sqrt(|q|^2) > MaxQ, decided on |q|^2 against the exact float threshold
+        const float2 s = f2add(f2add(mul(q0, q0), mul(q1, q1)), mul(q2, q2));
+        q0 = mul(q0, dup(a.vpdq));
+        q1 = mul(q1, dup(a.vpdq));
+        q2 = mul(q2, dup(a.vpdq));
+        if (DMAP) {  // first-level nearest neighbour: back to the voxel centre
+            auto near = [](float2 x) {
+                const float2 t = f2add(x, make_float2(copysignf(0.49999997f, x.x), copysignf(0.49999997f, x.y)));
+                return make_float2(truncf(t.x), truncf(t.y));
+            };
+            q0 = near(q0);
+            q1 = near(q1);
+            q2 = near(q2);
+        }
+        auto row = [&](float r0, float r1, float r2) {
+            return f2add(f2add(mul(q0, dup(r0)), mul(q1, dup(r1))), mul(q2, dup(r2)));
+        };
+        const float2 x0 = row(R[0], R[1], R[2]), x1 = row(R[3], R[4], R[5]), x2 = row(R[6], R[7], R[8]);
+        // the double product of two counts is exact, as the float one is
+        auto value = [&](float w) {
+            return SUM == SUM_VALUES ? d2u64(dmul(dmul((double)A.w, (double)w), a.mult))
+                                     : (unsigned long long)__float2uint_rz(fmul(A.w, w));
+        };
+        put_nearest<SUM>(a, s.x <= a.maxq2, x0.x, x1.x, x2.x, value(B0.w));
+        put_nearest<SUM>(a, s.y <= a.maxq2 && k + 1 < steps, x0.y, x1.y, x2.y, value(B1.w));
+    }
+}
+
+// Pairs of the fast path split over the eight voxels around their rotated q
+// (add_rotated<1>).  The values stay below 2^24, so their floor is read from the
+// low word of the double product rounded down to a multiple of one (an add of
+// 2^52 toward zero) instead of a 64-bit conversion.  A pair whose eight voxels
+// lie in the box adds there; of the others, neighbouring lanes exchange halves:
+// both lanes add one pair's two voxels of a mesh row, adjacent words, with one
+// instruction and then the other pair's, since L2 takes adjacent words of a
+// request together (measured: 3.4e11 adds/s in pairs, 2.2e11 single).
+template <int DMAP>
+__device__ __forceinline__ void linear_unit(const SparseArgs &a, const float4 *__restrict__ P, uint32_t n, const float *R,
+                                            uint32_t i, uint32_t d0, int steps, uint32_t L)
+{
+    const float4 A = ld_photon_hint(P + i, a.photon_policy);
+    const int odd = threadIdx.x & 1;
+    uint32_t j = i + d0;
+    if (j >= n) j -= n;
+    for (int k = 0; k < (int)L; k++) {  // all lanes: the exchange is warp-wide
+        const float4 B = ld_photon_hint(P + j, a.photon_policy);
+        const uint32_t flip = j < i ? 0x80000000u : 0u;  // q = k_lo - k_hi
+        j = j + 1 == n ? 0u : j + 1;
+        float q0 = fsub(A.x, B.x), q1 = fsub(A.y, B.y), q2 = fsub(A.z, B.z);
+        bool on = k < steps && fadd(fadd(fmul(q0, q0), fmul(q1, q1)), fmul(q2, q2)) <= a.maxq2;
+        auto scaled = [&](float q) {
+            q = fmul(__uint_as_float(__float_as_uint(q) ^ flip), a.vpdq);
+            return DMAP ? truncf(fadd(q, copysignf(0.49999997f, q))) : q;  // first level: the voxel centre
+        };
+        q0 = scaled(q0);
+        q1 = scaled(q1);
+        q2 = scaled(q2);
+        const float x0 = rot_row(q0, q1, q2, R[0], R[1], R[2]), x1 = rot_row(q0, q1, q2, R[3], R[4], R[5]),
+                    x2 = rot_row(q0, q1, q2, R[6], R[7], R[8]);
+        const double val = (double)fmul(A.w, B.w);  // exact: counts <= 128
+        const float m = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fabsf(x2));
+        if (on && !(m < (float)a.C)) {  // a voxel outside the mesh
+            add_rotated<1>(a, val, x0, x1, x2);
+            on = false;
+        }
+        const float f0 = floorf(x0), f1 = floorf(x1), f2 = floorf(x2);
+        const double sf = dsub(1.0, (double)fsub(x0, f0)), sm = dsub(1.0, (double)fsub(x1, f1)),
+                     sz = dsub(1.0, (double)fsub(x2, f2));
+        const double tm = dmul(val, a.mult);
+        const double yf[2] = {sm, dsub(1.0, sm)}, zf[2] = {sz, dsub(1.0, sz)}, xf[2] = {sf, dsub(1.0, sf)};
+        uint32_t v[4][2];  // [2 cz + cy][cx]
+#pragma unroll
+        for (int cy = 0; cy < 2; cy++)
+#pragma unroll
+            for (int cx = 0; cx < 2; cx++) {
+                const double w = dmul(xf[cx], yf[cy]);
+#pragma unroll
+                for (int cz = 0; cz < 2; cz++)
+                    v[2 * cz + cy][cx] = (uint32_t)__double2loint(__dadd_rz(dmul(tm, dmul(w, zf[cz])), 4503599627370496.0));
+            }
+        const int b0 = __float2int_rz(f0), b1 = __float2int_rz(f1), b2 = __float2int_rz(f2);
+        // the word of corner (cx, cy, cz) is the centre's plus its offset, or minus
+        // it for a negative slow index (the point reflection)
+        const bool in_box = on && m < a.box_lim - 0.5f;  // box_r: every corner within it
+        if (in_box) {
+            const int bl = b0 + b1 * (int)a.box_w + b2 * a.box_plane, ml = b0 + b1 * a.S + b2 * (int)a.plane;
+            uint32_t carry = 0;
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int cx = 0; cx < 2; cx++) {
+                    const int off = bl + (r & 1) * (int)a.box_w + (r >> 1) * a.box_plane + cx;
+                    const int at = a.box_center + (b2 + (r >> 1) < 0 ? -off : off);
+                    const uint32_t old = box_add32(a, (uint32_t)at, v[r][cx]);
+                    carry |= (old + v[r][cx] < old ? 1u : 0u) << (2 * r + cx);
+                }
+            while (carry) {
+                const int b = __ffs(carry) - 1, r = b >> 1;
+                carry &= carry - 1;
+                const int off = ml + (r & 1) * a.S + (r >> 1) * (int)a.plane + (b & 1), s = b2 + (r >> 1);
+                const uint32_t word = (uint32_t)(a.center + (s < 0 ? -off : off));
+                const uint32_t mirror = s == 0 ? 2u * (uint32_t)a.center - word : word;
+                carry_out(a.half, word, mirror, s == 0 && word == mirror ? 2u : 1u);
+            }
+        }
+        const bool in_mesh = on && !in_box;
+        if (__any_sync(0xffffffffu, in_mesh)) {
+            const int ml = b0 + b1 * a.S + b2 * (int)a.plane;
+            const int state = in_mesh ? b2 : -0x40000000;  // the partner's slow index, or nothing to add
+            const int pml = __shfl_xor_sync(0xffffffffu, ml, 1), pstate = __shfl_xor_sync(0xffffffffu, state, 1);
+            uint32_t own[4], got[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                own[r] = odd ? v[r][1] : v[r][0];
+                got[r] = __shfl_xor_sync(0xffffffffu, odd ? v[r][0] : v[r][1], 1);
+            }
+#pragma unroll
+            for (int turn = 0; turn < 2; turn++) {  // the even lane's pair, then the odd lane's
+                const bool mine = turn == odd;
+                const int base = (mine ? ml : pml) + odd, s0 = mine ? state : pstate;
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int off = base + (r & 1) * a.S + (r >> 1) * (int)a.plane, s = s0 + (r >> 1);
+                    const uint32_t word = (uint32_t)(a.center + (s < 0 ? -off : off));
+                    const uint32_t val32 = mine ? own[r] : got[r];
+                    if (s > -0x20000000 && val32) {
+                        mesh_add(a, word, val32);
+                        if (s == 0) mesh_add(a, 2u * (uint32_t)a.center - word, val32);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// threads of a CTA at most: all that share a box at 64 registers (linear second level: 680 us for
+// 3.6e7 pairs of a 129^3 mesh, 750 at 512 threads), fewer where 64 first-level corners each go on
+constexpr int pair_threads(int dmap, int i1, int i2) { return dmap && i1 ? 512 : 1024; }
+
+// One CTA per SM, whose warps take chunks of the batch (walk_share); its box of
+// the voxels around q = 0 takes their adds in shared memory and goes to the half
+// mesh once, at the end.  Bound by the L2 request rate of the adds outside the
+// box and by issue slots, about evenly: 89 instructions per 32 pairs (164 with
+// a thread per pair, its two loads and its index arithmetic), 100 000 frames
+// 4.2 ms (5.8 with a work queue, a barrier per frame and R = 9), one event of
+// 164 photons 8 us (three launches, 36 us), linear second level on 3.6e7 pairs
+// of a 129^3 mesh 0.67 ms (1.5).
+template <int DMAP, int I1, int I2>
+__global__ void __launch_bounds__(pair_threads(DMAP, I1, I2), 1) sparse_pairs_kernel(SparseArgs a)
+{
+    constexpr bool FAST = DMAP == 0 || I1 == 0;
+    __shared__ unsigned long long s_off[PAIR_DIRECT + 1];
+    __shared__ unsigned long long s_pairs;
+    __shared__ uint32_t s_next, s_taken, s_worst[32];
+    __shared__ uint32_t s_flags[PAIR_DIRECT];
+    extern __shared__ uint32_t s_box[];  // (box_r + 1) x box_w x box_w low words, [ss][ms][fs]
+    a.mesh_policy = a.cache_hints ? l2_policy_evict_last() : l2_policy_normal();
+    a.photon_policy = a.cache_hints ? l2_policy_evict_first() : l2_policy_normal();
     const uint32_t nthr = blockDim.x;
-    const uint32_t box_n = a.box_r ? (uint32_t)(a.box_r + 1) * a.box_w * a.box_w : 0u;
-    a.box_base = (uint32_t)__cvta_generic_to_shared(s_box);
-    a.box_hi = a.box_base + 4u * box_n;
-    for (uint32_t k = threadIdx.x; k < 2 * box_n; k += nthr) s_box[k] = 0u;  // visible after the
-                                                                            // loop's first barrier
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned long long t = atomicAdd(a.queue, 1ull);
-            s_tile = t;
-            if (t < ntiles) {
-                // last frame f with tile_off[f] <= t
-                uint32_t lo = 0, hi = a.nframes;  // tile_off[lo] <= t < tile_off[hi]
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (a.tile_off[mid] <= t)
-                        lo = mid;
-                    else
-                        hi = mid;
-                }
-                s_frame = lo;
-                s_small = a.small_counts ? a.small_counts[lo] : 0;
-#pragma unroll
-                for (int k = 0; k < 9; k++) s_rot[k] = a.rot[9 * (size_t)lo + k];
-            }
-        }
+    const int lane = threadIdx.x & 31;
+    const unsigned long long *off = a.walk.head ? a.walk.cost_off : s_off;
+    const PlanHeader h = a.walk.head ? *a.walk.head : plan_direct(a.walk, gridDim.x * (nthr / 32), s_off, &s_pairs);
+    const Share share = cta_share(h, a.walk.head != nullptr);
+    if (share.x0 >= share.x1) return;  // a CTA without work (uniform over the block)
+    if (threadIdx.x == 0) s_next = s_taken = 0u;
+    uint32_t worst = 0;  // the largest flag of the batch
+    if (FAST && a.fast_ok && a.check_here) {  // the planner's check, for the frames of this CTA
+        for (uint32_t f = threadIdx.x; f < a.walk.nframes; f += nthr) s_flags[f] = 1u;
         __syncthreads();
-        const unsigned long long t = s_tile;
-        if (t >= ntiles) break;
-        const uint32_t f = s_frame;
-        const bool small = s_small != 0;
-        float R[9];
-#pragma unroll
-        for (int k = 0; k < 9; k++) R[k] = s_rot[k];
-        const uint64_t base = a.offsets[f];
-        const uint32_t n = (uint32_t)(a.offsets[f + 1] - base);
-        const unsigned long long chunk = t - a.tile_off[f];
-        const float4 *__restrict__ P = a.photons + base;
-
-        // self pairs (q = 0): once per frame, on its first tile
-        if (chunk == 0) {
-            unsigned long long s = 0;
-            for (uint32_t i = threadIdx.x; i < n; i += nthr) {
-                const double v = (double)P[i].w;
-                s += d2u64(dmul(dmul(v, v), a.mult));
-            }
-            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if ((threadIdx.x & 31) == 0) s_self[threadIdx.x >> 5] = s;
+        for (uint32_t f = 0; f < a.walk.nframes; f++) {
+            if (off[f + 1] <= share.x0 || off[f] >= share.x1) continue;
+            const uint64_t b = a.walk.offsets[f], e = a.walk.offsets[f + 1];
+            uint32_t m = threadIdx.x >= 3 || fast_row(a.rot + 9 * (size_t)f + 3 * threadIdx.x, a.row_limit2) ? 1u : FLAG_GENERAL;
+            for (uint64_t i = b + threadIdx.x; i < e; i += nthr) m = max(m, fast_count(a.walk.photons[i]));
+            if (m > 128u) atomicMax(&s_flags[f], m);
+            worst = max(worst, m);
         }
-
-        // distinct pairs of this tile
-        const unsigned long long npairs = (unsigned long long)n * (n - 1) / 2;
-        const unsigned long long p0 = chunk * a.tile_pairs;
-        const unsigned long long p1 = min(npairs, p0 + a.tile_pairs);
-        if (p0 + threadIdx.x < p1) {
-            unsigned long long l = p0 + threadIdx.x;
-            uint32_t d = (uint32_t)(l / n) + 1;
-            uint32_t i = (uint32_t)(l - (unsigned long long)(d - 1) * n);
-            const uint32_t dq = nthr / n, dr = nthr % n;
-            for (; l < p1; l += nthr) {
-                uint32_t j = i + d;
-                if (j >= n) j -= n;
-                const uint32_t lo = min(i, j), hi = max(i, j);
-                if (a.cache_hints)
-                    bin_pair<DMAP, I1, I2>(a, ld_photon_hint(P + lo, photon_policy),
-                                           ld_photon_hint(P + hi, photon_policy), R, small);
-                else
-                    bin_pair<DMAP, I1, I2>(a, P[lo], P[hi], R, small);
-                i += dr;
-                d += dq;
-                if (i >= n) {
-                    i -= n;
-                    d += 1;
-                }
-            }
+    } else if (FAST && a.fast_ok) {
+        const uint32_t words = a.walk.nframes / 16;
+        const uint4 *fl = reinterpret_cast<const uint4 *>(a.flags);
+        uint32_t most = 0, least = 0xffffffffu;  // of the bytes
+        for (uint32_t k = threadIdx.x; k < words; k += nthr) {
+            const uint4 x = fl[k];
+            most = __vmaxu4(__vmaxu4(most, __vmaxu4(x.x, x.y)), __vmaxu4(x.z, x.w));
+            least = __vminu4(__vminu4(least, __vminu4(x.x, x.y)), __vminu4(x.z, x.w));
         }
-        __syncthreads();
-        if (chunk == 0 && threadIdx.x == 0) {
-            unsigned long long s = 0;
-            for (uint32_t w = 0; w < (nthr + 31) / 32; w++) s += s_self[w];
-            if (s) {  // q = 0: the box's centre when there is a box
-                if (a.box_r)
-                    box_add(a, (uint32_t)(a.box_r * a.box_w + a.box_r), s);
-                else
-                    atomicAdd(&a.half[(size_t)a.C + (size_t)a.C * a.S], s);
-            }
+        for (uint32_t f = 16 * words + threadIdx.x; f < a.walk.nframes; f += nthr) {
+            most = __vmaxu4(most, a.flags[f]);
+            least = __vminu4(least, 0xffffff00u | a.flags[f]);
+        }
+        for (int k = 0; k < 32; k += 8) {
+            worst = max(worst, (most >> k) & 255u);
+            if (((least >> k) & 255u) == 0) worst = FLAG_GENERAL;
         }
     }
-    // the loop ends after a barrier: every shared-memory add is done; flush the box
+    worst = __reduce_max_sync(0xffffffffu, worst);
+    if (lane == 0) s_worst[threadIdx.x >> 5] = worst;
+    // the box pays where its voxels collect many adds per CTA: its flush costs
+    // one coalesced mesh add per voxel
+    a.box_r = h.pairs < BOX_PAIRS_SMALL ? -1 : h.pairs < BOX_PAIRS_LARGE ? min(a.box_max, BOX_R_SMALL) : a.box_max;
+    a.box_w = a.box_r >= 0 ? 2u * a.box_r + 1u : 0u;
+    a.box_plane = (int)(a.box_w * a.box_w);
+    a.box_center = a.box_r >= 0 ? a.box_r + a.box_r * (int)a.box_w : 0;
+    a.box_lim = a.box_r >= 0 ? (float)a.box_r + 0.5f : 0.0f;
+    a.center = a.C + a.C * a.S;
+    a.box_base = (uint32_t)__cvta_generic_to_shared(s_box);
+    const uint32_t box_n = (uint32_t)(a.box_r + 1) * a.box_w * a.box_w;
+    for (uint32_t k = threadIdx.x; k < box_n; k += nthr) s_box[k] = 0u;
+    __syncthreads();
+    for (uint32_t w = 0; w < nthr / 32; w++) worst = max(worst, s_worst[w]);
+    // 32 pairs per unit of cost; a chunk's last unit may reach past it
+    const bool counts = FAST && I2 == 0 && a.fast_ok && a.mult_u && worst <= 128u &&
+                        (unsigned long long)share.most * (share.chunk + h.steps + PAIR_UNIT_COST) * 32 * (worst * worst) <
+                            (1ull << 32);
+
+    float R[9];
+    const float4 *__restrict__ P = nullptr;
+    uint32_t n = 0;
+    uint32_t flag = FLAG_GENERAL;
+    unsigned long long self = 0;  // self pairs (q = 0) of this lane
+    walk_share(
+        a.walk, h, off, share, a.walk.head ? &a.walk.head->next : &s_next, &s_taken,
+        [&](uint32_t f, uint64_t base, uint32_t nf) {
+            P = a.walk.photons + base;
+            n = nf;
+            if (FAST && a.fast_ok) {
+                flag = a.check_here ? s_flags[f] : a.flags[f];
+                if (flag == 0) flag = FLAG_GENERAL;
+                if (flag <= 128u && !a.mult_u) flag = FLAG_VALUES;
+            }
+#pragma unroll
+            for (int k = 0; k < 9; k++) R[k] = a.rot[9 * (size_t)f + k];
+        },
+        [&](uint32_t i, uint32_t c, bool active, uint32_t nc, uint32_t L) {
+            uint32_t d0;
+            int steps;
+            chunk_steps(n, i, c, L, active, d0, steps);
+            if (active && c == 0) {
+                const double v = (double)P[i].w;
+                self += d2u64(dmul(dmul(v, v), a.mult));
+            }
+            if (FAST && I2 && flag <= 128u) {
+                linear_unit<DMAP>(a, P, n, R, i, d0, steps, L);
+            } else if (FAST && !I2 && counts) {
+                nearest_unit<DMAP, SUM_COUNTS>(a, P, n, R, i, d0, steps);
+            } else if (FAST && !I2 && flag <= 128u) {
+                nearest_unit<DMAP, SUM_SMALL>(a, P, n, R, i, d0, steps);
+            } else if (FAST && !I2 && flag == FLAG_VALUES) {
+                nearest_unit<DMAP, SUM_VALUES>(a, P, n, R, i, d0, steps);
+            } else {
+                uint32_t j = i + d0;
+                if (j >= n) j -= n;
+                for (int k = 0; k < steps; k++) {
+                    bin_pair<DMAP, I1, I2>(a, P[min(i, j)], P[max(i, j)], R);
+                    if (++j == n) j = 0;
+                }
+            }
+        });
+    for (int o = 16; o; o >>= 1) self += __shfl_xor_sync(0xffffffffu, self, o);
+    if (lane == 0 && self) mesh_add(a, (uint32_t)a.C + (uint32_t)a.C * (uint32_t)a.S, self);
+    __syncthreads();
     for (uint32_t k = threadIdx.x; k < box_n; k += nthr) {
-        const unsigned long long v = split_word(s_box, s_box + box_n, k);
+        const unsigned long long v = counts ? (unsigned long long)s_box[k] * a.mult_u : s_box[k];
         if (v == 0) continue;
-        const uint32_t ss = k / (uint32_t)(a.box_w * a.box_w), r = k - ss * (uint32_t)(a.box_w * a.box_w);
-        const uint32_t ms = (uint32_t)(a.C - a.box_r) + r / (uint32_t)a.box_w;
-        const uint32_t fs = (uint32_t)(a.C - a.box_r) + r % (uint32_t)a.box_w;
-        unsigned long long *addr = &a.half[fs + ms * (uint32_t)a.S + ss * a.plane];
-        if (a.cache_hints)
-            red_add_hint(addr, v, a.mesh_policy);
-        else
-            atomicAdd(addr, v);
+        const uint32_t ss = k / (a.box_w * a.box_w), r = k - ss * (a.box_w * a.box_w);
+        const uint32_t ms = (uint32_t)(a.C - a.box_r) + r / a.box_w;
+        const uint32_t fs = (uint32_t)(a.C - a.box_r) + r % a.box_w;
+        const uint32_t word = fs + ms * (uint32_t)a.S + ss * a.plane;
+        mesh_add(a, word, v);
+        if (ss == 0) mesh_add(a, 2u * (uint32_t)a.center - word, v);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// planner: tiles per frame, exclusive scan, queue reset (one CTA)
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ unsigned long long frame_tiles(const uint64_t *off, uint32_t f,
+                                                          uint32_t tile_pairs)
+{
+    const unsigned long long n = off[f + 1] - off[f];
+    if (n == 0) return 0;
+    const unsigned long long pairs = n * (n - 1) / 2;
+    const unsigned long long t = (pairs + tile_pairs - 1) / tile_pairs;
+    return t > 0 ? t : 1;
+}
+
+__global__ void __launch_bounds__(PLAN_THREADS)
+    ac1d_plan_kernel(const uint64_t *__restrict__ off, uint32_t nframes, uint32_t tile_pairs,
+                       unsigned long long *__restrict__ tile_off, unsigned long long *queue)
+{
+    __shared__ unsigned long long warp_sums[PLAN_THREADS / 32];
+    const uint32_t tid = threadIdx.x;
+    const uint32_t chunk = (nframes + PLAN_THREADS - 1) / PLAN_THREADS;
+    const uint32_t f0 = min(nframes, tid * chunk), f1 = min(nframes, f0 + chunk);
+    unsigned long long local = 0;
+    for (uint32_t f = f0; f < f1; f++) local += frame_tiles(off, f, tile_pairs);
+    // block-wide exclusive scan of the per-thread sums
+    const int lane = tid & 31, w = tid >> 5;
+    unsigned long long incl = local;
+    for (int o = 1; o < 32; o <<= 1) {
+        unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_sums[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+        unsigned long long v = warp_sums[lane];
+        unsigned long long s = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            unsigned long long u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        warp_sums[lane] = s - v;  // exclusive warp prefix
+    }
+    __syncthreads();
+    unsigned long long run = warp_sums[w] + incl - local;
+    for (uint32_t f = f0; f < f1; f++) {
+        tile_off[f] = run;
+        run += frame_tiles(off, f, tile_pairs);
+    }
+    if (tid == PLAN_THREADS - 1) {
+        tile_off[nframes] = warp_sums[w] + incl;
+        *queue = 0ull;
     }
 }
 
@@ -525,6 +1054,14 @@ __device__ __forceinline__ uint32_t wrap_bin(uint32_t b, uint32_t n)
 }
 
 struct AC1DArgs {
+    const float4 *__restrict__ photons;
+    const uint64_t *__restrict__ offsets;
+    const unsigned long long *__restrict__ tile_off;  // nframes + 1
+    unsigned long long *queue;
+    DeviceCounters *counters;
+    uint32_t nframes;
+    uint32_t tile_pairs;
+    double mult;
     float maxq, dqdx;
     uint32_t vecsize;   // device-route bins (VecSize)
     uint32_t size;      // host-route bins (Shape.Size; 0 when no frame takes the host route)
@@ -544,11 +1081,11 @@ struct AC1DHist {
 };
 
 // host-route value v (>= 0) into bin b
-__device__ __forceinline__ void host_route_add(const SparseArgs &a, const AC1DArgs &b, const AC1DHist &h,
+__device__ __forceinline__ void host_route_add(const AC1DArgs &b, const AC1DHist &h,
                                                uint32_t bin, float v)
 {
     if (bin >= b.size) {  // only for inconsistent MaxQ / dq; the reference writes out of bounds
-        atomicAdd(&a.counters->out_of_mesh, 1ull);
+        atomicAdd(&b.counters->out_of_mesh, 1ull);
         return;
     }
     if (v == 0.0f) return;
@@ -567,9 +1104,10 @@ __device__ __forceinline__ void host_route_add(const SparseArgs &a, const AC1DAr
 }
 
 template <int INTERP>
-__global__ void __launch_bounds__(256) ac1d_sparse_kernel(const SparseArgs a, const AC1DArgs b)
+__global__ void __launch_bounds__(256) ac1d_sparse_kernel(const AC1DArgs a)
 {
     extern __shared__ unsigned long long hist[];
+    const AC1DArgs &b = a;
     AC1DHist h;
     h.dev_lo = reinterpret_cast<uint32_t *>(hist);
     h.dev_hi = h.dev_lo + b.vecsize;
@@ -611,7 +1149,7 @@ __global__ void __launch_bounds__(256) ac1d_sparse_kernel(const SparseArgs a, co
             for (uint32_t i = threadIdx.x; i < n; i += nthr) {
                 const float w = P[i].w;
                 if (host) {
-                    host_route_add(a, b, h, 0, fmul(2.0f, fmul(w, w)));
+                    host_route_add(b, h, 0, fmul(2.0f, fmul(w, w)));
                 } else {
                     const double v = (double)w;
                     const unsigned long long u = d2u64(dmul(dmul(v, v), a.mult));
@@ -640,13 +1178,13 @@ __global__ void __launch_bounds__(256) ac1d_sparse_kernel(const SparseArgs a, co
                             // (uint)floor(q + 0.5) in double, as floor(fl(q + 0.49999997f)) for q < 2^23
                             uint32_t iq;
                             floor_small(fadd(q, 0.49999997f), iq);
-                            host_route_add(a, b, h, iq, fmul(2.0f, pv));
+                            host_route_add(b, h, iq, fmul(2.0f, pv));
                         } else {
                             uint32_t iq;  // q = |q| / dq <= MaxQ / dq < 2^23
                             const float fq = floor_small(q, iq);
                             const float sep = fsub(q, fq);
-                            host_route_add(a, b, h, iq, fmul(2.0f, fmul(pv, fsub(1.0f, sep))));
-                            host_route_add(a, b, h, iq + 1, fmul(2.0f, fmul(pv, sep)));
+                            host_route_add(b, h, iq, fmul(2.0f, fmul(pv, fsub(1.0f, sep))));
+                            host_route_add(b, h, iq + 1, fmul(2.0f, fmul(pv, sep)));
                         }
                     } else {
                         const double val = dmul((double)A.w, (double)B.w);
@@ -733,7 +1271,7 @@ static iac_sparse_tuning effective_tuning(iac_ctx *ctx, uint32_t size_ab)
     }
     if (t.tile_pairs == 0) t.tile_pairs = 4096;
     if (t.block_threads == 0) t.block_threads = 256;
-    if (t.ctas_per_sm == 0) t.ctas_per_sm = 8;
+    if (t.ctas_per_sm == 0) t.ctas_per_sm = 4;
     return t;
 }
 
@@ -769,85 +1307,93 @@ static iac_status check_params(const iac_sparse_params *p)
     return IAC_OK;
 }
 
-// Half-width R of the shared-memory box of voxels around q = 0 (ss <= R,
-// |fs - C| <= R, |ms - C| <= R) that each CTA of the pair kernel accumulates
-// privately and adds to the half mesh once, when it runs out of tiles.  Pair
-// density peaks at q = 0: in a 201^3 mesh of the rotated workload the
-// R = 10 box (4 851 voxels) takes 9 % of all updates, and without it those
-// few hundred 128-byte lines are the most contended L2 atomic targets (one
-// line takes about 4.5e9 atomic adds per second, the whole L2 about 1.9e11).
-// R = IAC_PAIR_BOX_R (10: 38 KB per CTA) while ctas_per_sm boxes fit in
-// 200 KB of the SM's shared memory, smaller beyond; at most C.
-#ifndef IAC_PAIR_BOX_R
-#define IAC_PAIR_BOX_R 10
-#endif
-static int pair_box_radius(int C, uint32_t ctas_per_sm)
+// The launch shape of a tuning setting: the threads that block_threads x
+// ctas_per_sm asks for on an SM, in as few CTAs as hold them, since the warps
+// of one CTA share one box and a larger box keeps more adds out of L2.
+struct PairShape {
+    int ctas, threads;  // per SM, per CTA
+    int box_max;
+};
+static PairShape pair_shape(const iac_sparse_tuning &tun, int max_threads, int C)
 {
-    const size_t budget = (200u << 10) / std::max<uint32_t>(1, ctas_per_sm);
-    int r = std::min(IAC_PAIR_BOX_R, C);
-    while (r > 0 && sizeof(unsigned long long) * (size_t)(r + 1) * (2 * r + 1) * (2 * r + 1) > budget) r--;
-    return r;
+    const int total = (int)(tun.block_threads * tun.ctas_per_sm);
+    PairShape s;
+    s.ctas = (total + max_threads - 1) / max_threads;
+    s.threads = std::max(32, std::min(max_threads, (total / s.ctas + 31) / 32 * 32));
+    const int budget = (184 << 10) / s.ctas;
+    s.box_max = std::min(BOX_R_MAX, C);
+    while (s.box_max >= 0 && 4 * (s.box_max + 1) * (2 * s.box_max + 1) * (2 * s.box_max + 1) > budget) s.box_max--;
+    return s;
 }
 
-// Work-queue memory of one batch: tile table (nframes + 1), queue counter,
-// per-frame small-count flags (nframes bytes).
+// Work-queue memory of one batch: planner header, table of frame starts
+// (nframes + 1), per-frame flags (nframes bytes).
 struct QueueMem {
-    unsigned long long *tile_off;
-    unsigned long long *queue;
+    unsigned long long *cost_off;
+    PlanHeader *head;
     unsigned char *flags;
 };
 
-// Planner, count check and pair kernel of one batch into the half mesh d_half.
+// Planner with its count check, and pair kernel of one batch into the half mesh
+// d_half.  Batches of up to PAIR_DIRECT frames are planned by the pair kernel's
+// own CTAs in shared memory: a live event is one launch instead of three.
 static iac_status launch_pair_batch(iac_ctx *ctx, const float *d_photons, const uint64_t *d_off,
                                     const float *d_rot9, uint32_t nframes, const iac_sparse_params *p,
                                     const QueueMem &q, uint64_t *d_half, cudaStream_t s)
 {
     const iac_sparse_tuning tun = effective_tuning(ctx, p->shape.size_ab);
-    sparse_plan_kernel<<<1, PLAN_THREADS, 0, s>>>(d_off, nframes, tun.tile_pairs, q.tile_off, q.queue);
-    IAC_LAUNCHED(ctx);
-    IAC_CUDA(cudaGetLastError());
-    const bool mult_small_int = p->multiplicator >= 1.0 && p->multiplicator <= 1024.0 &&
-                                p->multiplicator == std::floor(p->multiplicator);
-    unsigned char *flags = nullptr;
-    if (mult_small_int && p->interp_second == 0 && !(p->double_map && p->interp_first == 1)) {
-        const uint32_t blocks = (uint32_t)(((uint64_t)nframes * 32 + 255) / 256);
-        sparse_count_check_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const float4 *>(d_photons),
-                                                         d_off, nframes, q.flags);
-        IAC_LAUNCHED(ctx);
-        IAC_CUDA(cudaGetLastError());
-        flags = q.flags;
-    }
-    SparseArgs a;
-    a.photons = reinterpret_cast<const float4 *>(d_photons);
-    a.offsets = d_off;
+    const int i1 = p->double_map ? p->interp_first : 0;
+    const int C = ((int)p->shape.size_ab - 1) / 2;
+    const PairShape sh = pair_shape(tun, pair_threads(p->double_map, i1, p->interp_second), C);
+    const int grid = ctx->sm_count * sh.ctas;
+    const bool direct = nframes <= PAIR_DIRECT;
+    SparseArgs a{};
+    a.walk.photons = reinterpret_cast<const float4 *>(d_photons);
+    a.walk.offsets = d_off;
+    a.walk.head = direct ? nullptr : q.head;
+    a.walk.cost_off = q.cost_off;
+    a.walk.nframes = nframes;
+    a.walk.steps_max = std::min(PAIR_STEPS_MAX, std::max(1u, tun.tile_pairs / 32));
     a.rot = d_rot9;
-    a.tile_off = q.tile_off;
     a.half = reinterpret_cast<unsigned long long *>(d_half);
-    a.queue = q.queue;
     a.counters = ctx->d_counters;
-    a.nframes = nframes;
-    a.tile_pairs = tun.tile_pairs;
     a.S = (int)p->shape.size_ab;
-    a.C = (a.S - 1) / 2;
+    a.C = C;
     a.half_ss = (a.S + 1) / 2;
     a.plane = (uint32_t)a.S * (uint32_t)a.S;
-    a.maxq = p->shape.max_q;
     a.maxq2 = sqrt_threshold(p->shape.max_q);
     a.vpdq = (float)p->shape.voxel_per_dq;
+    a.neg_zero = -0.0f;
     a.mult = p->multiplicator;
-    a.mult_f = (float)p->multiplicator;
-    a.small_counts = flags;
+    a.mult_u = p->multiplicator >= 1.0 && p->multiplicator <= 1024.0 &&
+                       p->multiplicator == std::floor(p->multiplicator)
+                   ? (uint32_t)p->multiplicator
+                   : 0u;
+    a.fast_ok = std::isfinite(a.maxq2);
+    a.check_here = direct ? 1 : 0;
+    a.flags = q.flags;
     a.cache_hints = tun.cache_hints == 1 ? 1 : 0;
-    a.mesh_policy = 0;
-    a.box_r = pair_box_radius(a.C, tun.ctas_per_sm);
-    a.box_w = 2 * a.box_r + 1;
-    a.box_base = 0;
-    a.box_hi = 0;
-    const size_t box_bytes = a.box_r ? sizeof(unsigned long long) * (a.box_r + 1) * a.box_w * a.box_w : 0;
+    a.box_max = sh.box_max;
+    // |x| <= |row| (MaxQ Voxel_per_dq + the first level's rounding) < C + 1/2, with a margin for FP32
+    const double reach = ((double)p->shape.max_q * p->shape.voxel_per_dq + 0.8661) * 1.00001;
+    const double limit = ((double)C + 0.49) / reach;
+    a.row_limit2 = std::isfinite(limit) ? (float)(limit * limit * 0.99999) : -1.0f;
+    if (p->interp_second) a.row_limit2 = 1e12f;  // the linear path looks at every pair
+    if (!direct) {
+        const unsigned check = std::min<unsigned>((nframes + PLAN_THREADS / 32 - 1) / (PLAN_THREADS / 32),
+                                                  2u * (unsigned)ctx->sm_count);
+        const unsigned ctas = PLAN_CTAS + (check + PLAN_CTAS - 1) / PLAN_CTAS * PLAN_CTAS;
+        sparse_plan_kernel<<<ctas, PLAN_THREADS, 0, s>>>(d_off, nframes, a.walk.steps_max,
+                                                         (uint32_t)(grid * sh.threads / 32), q.cost_off, q.head,
+                                                         a.walk.photons, d_rot9, a.row_limit2, q.flags);
+        IAC_LAUNCHED(ctx);
+        IAC_CUDA(cudaGetLastError());
+    }
+    const size_t box_bytes = sizeof(uint32_t) * (size_t)(sh.box_max + 1) * (2 * sh.box_max + 1) * (2 * sh.box_max + 1);
     const PairKernel k = pick_kernel(p->double_map, p->interp_first, p->interp_second);
-    if (box_bytes > (48u << 10))
+    if (box_bytes > (40u << 10))
         IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)box_bytes));
-    k<<<ctx->sm_count * (int)tun.ctas_per_sm, tun.block_threads, box_bytes, s>>>(a);
+    k<<<grid, sh.threads, box_bytes, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
     return IAC_OK;
@@ -866,10 +1412,10 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
     unsigned long long *tile_off = (unsigned long long *)scratch;
     unsigned long long *queue = (unsigned long long *)((char *)scratch + table_bytes);
     cudaStream_t s = as_stream(stream);
-    sparse_plan_kernel<<<1, PLAN_THREADS, 0, s>>>(d_off, nframes, tun.tile_pairs, tile_off, queue);
+    ac1d_plan_kernel<<<1, PLAN_THREADS, 0, s>>>(d_off, nframes, tun.tile_pairs, tile_off, queue);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
-    SparseArgs a{};
+    AC1DArgs a = b;
     a.photons = reinterpret_cast<const float4 *>(d_photons);
     a.offsets = d_off;
     a.tile_off = tile_off;
@@ -883,7 +1429,7 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
     IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // as many persistent CTAs as fit: four per SM, fewer when the histograms are large
     const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (200u << 10) / std::max<size_t>(smem, 1)));
-    k<<<ctx->sm_count * per_sm, 256, smem, s>>>(a, b);
+    k<<<ctx->sm_count * per_sm, 256, smem, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
     return IAC_OK;
@@ -933,7 +1479,7 @@ iac_status iac_sparse_ac_batch(iac_ctx *ctx, const float *d_photons, const uint6
     const size_t table_bytes = ((sizeof(unsigned long long) * ((size_t)nframes + 1) + 127) / 128) * 128;
     st = stream_scratch(ctx, stream, SLOT_TILES, table_bytes + 128 + nframes, &scratch);
     if (st != IAC_OK) return st;
-    const QueueMem q{(unsigned long long *)scratch, (unsigned long long *)((char *)scratch + table_bytes),
+    const QueueMem q{(unsigned long long *)scratch, (PlanHeader *)((char *)scratch + table_bytes),
                      (unsigned char *)scratch + table_bytes + 128};
     return launch_pair_batch(ctx, d_photons, d_off, d_rot9, nframes, p, q, d_half, as_stream(stream));
 }
@@ -1271,7 +1817,7 @@ extern "C" iac_status iac_sparse_ac_batch_static(iac_ctx *ctx, const float *d_ph
     IAC_REQUIRE(ctx->static_scratch != nullptr, "iac_sparse_ac_batch_static: the context has no fixed scratch");
     DeviceGuard g(ctx->device);
     char *base = (char *)ctx->static_scratch;
-    const QueueMem q{(unsigned long long *)base, (unsigned long long *)(base + STATIC_TABLE_BYTES),
+    const QueueMem q{(unsigned long long *)base, (PlanHeader *)(base + STATIC_TABLE_BYTES),
                      (unsigned char *)base + STATIC_TABLE_BYTES + STATIC_QUEUE_BYTES};
     return launch_pair_batch(ctx, d_photons, d_off, d_rot9, nframes, p, q, d_half, as_stream(stream));
 }
