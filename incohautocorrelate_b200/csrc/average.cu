@@ -23,10 +23,12 @@
 //   photon_means_kernel    MeanIntensity / PhotonCount from those totals: the
 //                          values are integers, so while a frame's total stays
 //                          below 2^24 its sequential FP32 sum is that total;
-//   frame_sums_kernel      the sequential FP32 sum in pixel order, a lane per
-//                          frame fed by warps that stream and process the
-//                          pixels: for every frame without discretisation and
-//                          for frames of 2^24 photons or more.
+//   frame_scan_kernel      the sequential FP32 sum in pixel order as integer
+//                          sums, a CTA per frame: for frames without discretisation
+//                          and for frames of 2^24 photons or more;
+//   frame_sums_kernel      the same sum as a chain of adds, a lane per frame fed
+//                          by warps that stream and process the pixels: for short
+//                          frames.
 #include <algorithm>
 #include <cmath>
 
@@ -185,6 +187,247 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity)
     return false;
 }
 
+// A frame's value of one pixel as the reference sums it: masked, then thresholded
+// or discretised to photons.
+__device__ __forceinline__ float frame_value(float t, bool masked, int m, float thr, float step)
+{
+    if (masked) t = fmul(t, (float)m);
+    if (step > 0.0f) return t >= thr ? ceilf(__fdiv_rn(fsub(t, thr), step)) : 0.0f;
+    return (thr > 0.0f && t < thr) ? 0.0f : t;
+}
+
+// The sequential FP32 sum of a frame in pixel order, without its chain of
+// dependent adds.  While the sum stays within one binade, |sum| = A u with u its
+// last place and A an integer in [2^23, 2^24), adding x rounds to A + rint(x / u):
+// the increments are integers that depend on x alone, so they add up in any
+// order, with two exceptions that are looked for.  A tie (x / u half way between
+// integers) rounds to an even A, so its increment depends on the parity of A
+// before it; and a sum that leaves the binade changes u.  A chunk of SCAN_PIX
+// pixels without ties, whose positive and negative increments together cannot
+// leave the binade, is one block sum (SCAN_PIX = SCAN_RUN pixels per thread).  Any other chunk is laid out in pixel order
+// in shared memory; a run of pixels is then a map from
+// the parity before it to its increment, and maps compose, so an ordered scan
+// over the threads gives every thread its exact A; the first thread that may
+// leave the binade adds its pixels one by one, and the scan goes on behind it.
+// A sum starts with a few such rounds (the binade doubles with the pixel count)
+// and then meets a tie or a new binade every few chunks.  Where the rounds do not
+// get far (the first pixels, a sum that hovers around zero), the adding thread
+// takes more pixels each time, up to the whole chunk.
+// 300 frames of 1024 x 512 in 0.28 ms (frame_sums_kernel, the chain of adds:
+// 1.84 ms), 0.097 at the copy rate: bound by the latency of a chunk's block sum
+// and by the few ordered scans, with two or three frames per SM.
+constexpr int SCAN_RUN = 16;
+constexpr int SCAN_PITCH = SCAN_RUN + 1;  // a run per thread, without bank conflicts
+constexpr float SCAN_MAGIC = 12582912.0f;  // 1.5 * 2^23: z + SCAN_MAGIC rounds |z| < 2^22 to an integer
+
+// a run of pixels: its increment of A for an even and an odd A before it
+struct ParityMap {
+    int even, odd;
+};
+__device__ __forceinline__ ParityMap then(ParityMap a, ParityMap b)
+{
+    return {a.even + ((a.even & 1) ? b.odd : b.even), a.odd + ((a.odd & 1) ? b.even : b.odd)};
+}
+
+template <bool VEC, int SCAN_THREADS>
+__global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
+    frame_scan_kernel(const float *__restrict__ frames, uint64_t npix, const int *__restrict__ mask, float thr,
+                      float step, const int *__restrict__ only, float *__restrict__ mean, float *__restrict__ count)
+{
+    constexpr int WARPS = SCAN_THREADS / 32, SCAN_PIX = SCAN_THREADS * SCAN_RUN;
+    __shared__ float s_x[SCAN_THREADS * SCAN_PITCH];
+    __shared__ int s_red[2][WARPS][3];  // by chunk parity: increments, their sizes, needs the scan
+    __shared__ ParityMap s_map[WARPS];
+    __shared__ int s_first[WARPS];
+    __shared__ float s_acc;
+    const uint32_t f = blockIdx.x;
+    if (only && !only[f]) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const float *row = frames + (size_t)f * npix;
+    const bool masked = mask != nullptr;
+    // element e of this thread's SCAN_RUN within a chunk: rows of 16 bytes (VEC) or single pixels
+    auto slot = [&](int e) { return VEC ? (e / 4 * SCAN_THREADS + tid) * 4 + e % 4 : e * SCAN_THREADS + tid; };
+    float raw[SCAN_RUN];
+    int mk[SCAN_RUN];
+    auto load = [&](uint64_t p0) {
+#pragma unroll
+        for (int e = 0; e < SCAN_RUN; e += VEC ? 4 : 1) {
+            const uint64_t j = p0 + slot(e);
+            const bool in = j < npix;  // npix % 4 == 0 with VEC: four pixels are whole or absent
+            if constexpr (VEC) {
+                const float4 v = in ? __ldcs(reinterpret_cast<const float4 *>(row + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const int4 m = in && masked ? __ldg(reinterpret_cast<const int4 *>(mask + j)) : make_int4(0, 0, 0, 0);
+                raw[e] = v.x, raw[e + 1] = v.y, raw[e + 2] = v.z, raw[e + 3] = v.w;
+                mk[e] = m.x, mk[e + 1] = m.y, mk[e + 2] = m.z, mk[e + 3] = m.w;
+            } else {
+                raw[e] = in ? __ldcs(row + j) : 0.0f;
+                mk[e] = in && masked ? __ldg(mask + j) : 0;
+            }
+        }
+    };
+    float acc = 0.0f;  // the sum so far, the same in every thread
+    // the binade of acc: scale = sign / u, A = |acc| / u; false where it has none to work with
+    auto binade = [&](float &scale, int &A) {
+        const uint32_t b = __float_as_uint(acc);
+        const int e = (int)((b >> 23) & 255u);
+        A = (int)((b & 0x7fffffu) | 0x800000u);
+        if (e < 40 || e > 250) return false;
+        scale = __uint_as_float(((uint32_t)(277 - e) << 23) | (b & 0x80000000u));  // 2^(150 - e)
+        return true;
+    };
+    int runs = 1;  // that the adding thread takes; twice as many after a round that did not get as far
+    load(0);
+    for (uint64_t p0 = 0, c = 0; p0 < npix; p0 += SCAN_PIX, c++) {
+        float x[SCAN_RUN];
+#pragma unroll
+        for (int e = 0; e < SCAN_RUN; e++) x[e] = frame_value(raw[e], masked, mk[e], thr, step);
+        if (npix - p0 < SCAN_PIX) {  // pixels past the end add 0
+            const int left = (int)(npix - p0);
+#pragma unroll
+            for (int e = 0; e < SCAN_RUN; e++) x[e] = slot(e) < left ? x[e] : 0.0f;
+        }
+        if (npix - p0 > SCAN_PIX) load(p0 + SCAN_PIX);
+        float scale = 0.0f;
+        int A = 0;
+        const bool ok = binade(scale, A);
+        // the increments and their sizes as floats, exact while the sizes stay below
+        // 2^21 (anything too large for SCAN_MAGIC, infinite or NaN puts them past it)
+        int inc = 0, size = 0, scan = 0;
+        if (ok) {
+            float2 sum = make_float2(0.0f, 0.0f);
+            float fsize = 0.0f;
+            bool tie = false;
+#pragma unroll
+            for (int e = 0; e < SCAN_RUN; e += 2) {
+                const float2 z = f2mul(make_float2(x[e], x[e + 1]), make_float2(scale, scale));  // exact
+                const float2 r = f2sub(f2add(z, make_float2(SCAN_MAGIC, SCAN_MAGIC)), make_float2(SCAN_MAGIC, SCAN_MAGIC));
+                const float2 d = f2sub(z, r);
+                tie |= fabsf(d.x) == 0.5f || fabsf(d.y) == 0.5f;
+                sum = f2add(sum, r);
+                fsize = fadd(fadd(fsize, fabsf(r.x)), fabsf(r.y));
+            }
+            const bool far = !(fsize < 2097152.0f);
+            inc = __reduce_add_sync(0xffffffffu, far ? 0 : (int)fadd(sum.x, sum.y));
+            size = __reduce_add_sync(0xffffffffu, far ? 0 : (int)fsize);
+            scan = __any_sync(0xffffffffu, tie || far);
+        } else {
+            bool some = false;
+#pragma unroll
+            for (int e = 0; e < SCAN_RUN; e++) some |= !(x[e] == 0.0f);
+            scan = __any_sync(0xffffffffu, some);
+        }
+        int (*red)[3] = s_red[c & 1];
+        if (lane == 0) red[warp][0] = inc, red[warp][1] = size, red[warp][2] = scan;
+        __syncthreads();
+        int ti = 0, ts = 0, need = 0;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) ti += red[w][0], ts += red[w][1], need |= red[w][2];
+        const int up = (ts + ti) >> 1, down = (ts - ti) >> 1;
+        if (!need && (!ok || (A + up < (1 << 24) && A - down > (1 << 23)))) {
+            if (ok) acc = fmul((float)(A + ti), __uint_as_float((__float_as_uint(acc) & 0x80000000u) |
+                                                               ((((__float_as_uint(acc) >> 23) & 255u) - 23u) << 23)));
+            continue;
+        }
+        // ordered scan; s_x is free: every thread has passed the barrier above
+#pragma unroll
+        for (int e = 0; e < SCAN_RUN; e++) s_x[slot(e) / SCAN_RUN * SCAN_PITCH + slot(e) % SCAN_RUN] = x[e];
+        const float *own = s_x + tid * SCAN_PITCH;
+        for (int t0 = 0; t0 < SCAN_THREADS;) {
+            __syncthreads();  // s_x written, the previous round's results read
+            const bool good = binade(scale, A);
+            ParityMap m{0, 0};
+            int hi = 0, lo = 0, bad = 0;
+            if (tid >= t0) {
+                float sum = 0.0f, size = 0.0f, ties = 0.0f;
+                bool some = false;
+                const float by = good ? scale : 1.0f;
+#pragma unroll
+                for (int e = 0; e < SCAN_RUN; e++) {
+                    const float z = fmul(own[e], by), r = fsub(fadd(z, SCAN_MAGIC), SCAN_MAGIC);
+                    ties = fabsf(fsub(z, r)) == 0.5f ? fadd(ties, 1.0f) : ties;
+                    some |= !(z == 0.0f);
+                    sum = fadd(sum, r);
+                    size = fadd(size, fabsf(r));
+                }
+                bad = good ? !(size < 2097152.0f) : some;
+                if (!bad && good) {
+                    m = {(int)sum, (int)sum};
+                    const int s = (int)size + (int)ties;
+                    hi = (s + (int)sum) / 2 + (int)ties;
+                    lo = (s - (int)sum) / 2 + (int)ties;
+                    if (ties != 0.0f) {
+                        m = {0, 0};
+#pragma unroll 1
+                        for (int e = 0; e < SCAN_RUN; e++) {
+                            const float z = fmul(own[e], scale), r = fsub(fadd(z, SCAN_MAGIC), SCAN_MAGIC);
+                            const int k = (int)r, fl = r > z ? k - 1 : k;  // fl: a tie's lower neighbour
+                            // even A: to the even one of fl, fl + 1; odd A: to the odd one
+                            m = then(m, fabsf(fsub(z, r)) == 0.5f ? ParityMap{fl + (fl & 1), fl + 1 - (fl & 1)}
+                                                                  : ParityMap{k, k});
+                        }
+                    }
+                    if (some) lo = max(lo, 1);  // a negative value may round to no increment
+                }
+            }
+            ParityMap incl = m;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const ParityMap u{__shfl_up_sync(0xffffffffu, incl.even, o), __shfl_up_sync(0xffffffffu, incl.odd, o)};
+                if (lane >= o) incl = then(u, incl);
+            }
+            if (lane == 31) s_map[warp] = incl;
+            ParityMap before{__shfl_up_sync(0xffffffffu, incl.even, 1), __shfl_up_sync(0xffffffffu, incl.odd, 1)};
+            if (lane == 0) before = {0, 0};
+            __syncthreads();
+            ParityMap ahead{0, 0}, all{0, 0};
+            for (int w = 0; w < WARPS; w++) {
+                if (w == warp) ahead = all;
+                all = then(all, s_map[w]);
+            }
+            before = then(ahead, before);
+            const int start = A + ((A & 1) ? before.odd : before.even);
+            if (good) bad |= start + hi >= (1 << 24) || (lo > 0 && start - lo <= (1 << 23));
+            const unsigned b = __ballot_sync(0xffffffffu, bad);
+            if (lane == 0) s_first[warp] = b ? warp * 32 + __ffs(b) - 1 : SCAN_THREADS;
+            __syncthreads();
+            int first = SCAN_THREADS;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) first = min(first, s_first[w]);
+            const float unit = __uint_as_float((__float_as_uint(acc) & 0x80000000u) |
+                                               ((((__float_as_uint(acc) >> 23) & 255u) - 23u) << 23));
+            if (first == SCAN_THREADS) {
+                if (good) acc = fmul((float)(A + ((A & 1) ? all.odd : all.even)), unit);
+                break;
+            }
+            if (good) runs = first - t0 < runs ? min(2 * runs, SCAN_THREADS) : 1;
+            const int behind = min(SCAN_THREADS, first + (good ? runs : 32));
+            if (tid == first) {
+                float s = good ? fmul((float)start, unit) : acc;
+                float v[SCAN_RUN], next[SCAN_RUN];
+#pragma unroll
+                for (int e = 0; e < SCAN_RUN; e++) next[e] = own[e];
+                for (const float *run = own; run != s_x + behind * SCAN_PITCH;) {
+                    run += SCAN_PITCH;
+                    const float *ahead_of = run != s_x + behind * SCAN_PITCH ? run : own;
+#pragma unroll
+                    for (int e = 0; e < SCAN_RUN; e++) v[e] = next[e], next[e] = ahead_of[e];
+#pragma unroll
+                    for (int e = 0; e < SCAN_RUN; e++) s = fadd(s, v[e]);
+                }
+                s_acc = s;
+            }
+            __syncthreads();
+            acc = s_acc;
+            t0 = behind;
+        }
+        __syncthreads();  // s_x is read
+    }
+    if (tid == 0) {
+        mean[f] = __fdiv_rn(acc, (float)npix);
+        if (count) count[f] = acc;
+    }
+}
+
 // Sequential per-frame FP32 sums of FPC frames per CTA.  Warp SUM_WARP sums:
 // lane i < FPC adds frame f0 + i's processed values in pixel order, one
 // dependent add per pixel, which is the reference's sequential sum and the
@@ -268,11 +511,7 @@ __global__ void __launch_bounds__(32 * (SUM_WARP + 1)) frame_sums_kernel(
             }
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         };
-        auto process = [&](float t, float m) {
-            if (mask) t = fmul(t, m);
-            if (step > 0.0f) return t >= thr ? ceilf(__fdiv_rn(fsub(t, thr), step)) : 0.0f;
-            return (thr > 0.0f && t < thr) ? 0.0f : t;
-        };
+        auto process = [&](float t, int m) { return frame_value(t, mask != nullptr, m, thr, step); };
 #pragma unroll 1
         for (int k = 0; k < SUM_RAW - 1; k++) issue(k);
 #pragma unroll 1
@@ -286,11 +525,8 @@ __global__ void __launch_bounds__(32 * (SUM_WARP + 1)) frame_sums_kernel(
             const float *st = raw + (ch % SUM_RAW) * C::RAW_FLOATS;
             float *out = cooked + c * C::COOKED_FLOATS;
             if constexpr (VEC) {
-                float4 m = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-                if (mask) {
-                    const int4 mi = *reinterpret_cast<const int4 *>(st + (FPC + warp) * SUM_PITCH + 4 * lane);
-                    m = make_float4((float)mi.x, (float)mi.y, (float)mi.z, (float)mi.w);
-                }
+                int4 m = make_int4(1, 1, 1, 1);
+                if (mask) m = *reinterpret_cast<const int4 *>(st + (FPC + warp) * SUM_PITCH + 4 * lane);
 #pragma unroll
                 for (int i = 0; i < RPW; i++) {
                     const float4 v = *reinterpret_cast<const float4 *>(st + (r0 + i) * SUM_PITCH + 4 * lane);
@@ -300,7 +536,7 @@ __global__ void __launch_bounds__(32 * (SUM_WARP + 1)) frame_sums_kernel(
             } else {
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const float m = mask ? (float)__float_as_int(st[(FPC + warp) * SUM_PITCH + 32 * q + lane]) : 1.0f;
+                    const int m = mask ? __float_as_int(st[(FPC + warp) * SUM_PITCH + 32 * q + lane]) : 1;
 #pragma unroll
                     for (int i = 0; i < RPW; i++)
                         out[(r0 + i) * SUM_PITCH + 32 * q + lane] = process(st[(r0 + i) * SUM_PITCH + 32 * q + lane], m);
@@ -391,13 +627,37 @@ iac_status launch_sums_fpc(int sms, const float *frames, uint64_t npix, uint32_t
     return launch_sums<VEC, 4>(frames, npix, nframes, mask, thr, step, only, mean, count, ctr, s);
 }
 
-iac_status launch_frame_sums(int sms, const float *frames, uint64_t npix, uint32_t nframes, const int *mask,
-                             float thr, float step, const int *only, float *mean, float *count, DeviceCounters *ctr,
-                             cudaStream_t s)
+// The frames' sequential sums (only: those with a nonzero entry): as integer
+// sums, or as chains of adds where a frame is short, since the integer sums start
+// with some ten rounds of their ordered scan: frames of 100 x 100, 100 of them
+// 41 us (chains 56) but 1 000 of them 147 (121); frames of 200 x 200, 600 of them
+// 171 (225); one frame of 300 x 300 58 (325).  Frames without a signal, whose sums
+// hover around zero, are added nearly pixel by pixel either way (300 of 512 x 1024:
+// 2.1 ms, chains 1.9), so batches of many frames per SM, which the chains take 8 and
+// more to a CTA, stay with them (2 000 of 300 x 300: 0.62 ms, chains 0.74, but
+// without a signal 1.3 and 0.74).
+iac_status launch_frame_sums(iac_ctx *ctx, const float *frames, uint64_t npix, uint32_t nframes, const int *mask,
+                             float thr, float step, const int *only, float *mean, float *count, cudaStream_t s)
 {
     const bool vec = npix % 4 == 0 && ((uintptr_t)frames & 15) == 0 && ((uintptr_t)mask & 15) == 0;
-    return vec ? launch_sums_fpc<true>(sms, frames, npix, nframes, mask, thr, step, only, mean, count, ctr, s)
-               : launch_sums_fpc<false>(sms, frames, npix, nframes, mask, thr, step, only, mean, count, ctr, s);
+    const int sms = ctx->sm_count;
+    const bool scan = (npix >= 16384 && nframes <= 8u * sms) || (npix >= 8192 && nframes <= 2u * sms);
+    if (scan) {
+        // smaller CTAs once every SM has its two frames (2 000 frames of 300 x 300: 509 us
+        // with 128 threads, 608 with 256; 250 of 512 x 1024: 341 and 316)
+        const bool many = nframes > 2u * sms;
+        auto k = vec ? (many ? frame_scan_kernel<true, 128> : frame_scan_kernel<true, 256>)
+                     : (many ? frame_scan_kernel<false, 128> : frame_scan_kernel<false, 256>);
+        k<<<nframes, many ? 128 : 256, 0, s>>>(frames, npix, mask, thr, step, only, mean, count);
+        IAC_LAUNCHED(ctx);
+        IAC_CUDA(cudaGetLastError());
+        return IAC_OK;
+    }
+    const iac_status st =
+        vec ? launch_sums_fpc<true>(sms, frames, npix, nframes, mask, thr, step, only, mean, count, ctx->d_counters, s)
+            : launch_sums_fpc<false>(sms, frames, npix, nframes, mask, thr, step, only, mean, count, ctx->d_counters, s);
+    if (st == IAC_OK) IAC_LAUNCHED(ctx);
+    return st;
 }
 
 }  // namespace
@@ -450,20 +710,18 @@ iac_status iac_average_frames(iac_ctx *ctx, const float *d_frames, uint64_t npix
         IAC_LAUNCHED(ctx);
         IAC_CUDA(cudaGetLastError());
         // frames of 2^24 photons or more: the sequential sum in pixel order
-        st = launch_frame_sums(ctx->sm_count, d_frames, npix, nframes, d_mask, threshold, step, redo, d_mean_intensity,
-                               d_photon_sum, ctx->d_counters, s);
+        st = launch_frame_sums(ctx, d_frames, npix, nframes, d_mask, threshold, step, redo, d_mean_intensity,
+                               d_photon_sum, s);
         if (st != IAC_OK) return st;
-        IAC_LAUNCHED(ctx);
     } else {
         auto kern = vec ? average_pixels_kernel<true, false, false> : average_pixels_kernel<false, false, false>;
         kern<<<grid, PIX_THREADS, 0, s>>>(d_frames, npix, nframes, d_mask, threshold, step, 0.0f, d_sum, discr,
                                           nullptr);
         IAC_LAUNCHED(ctx);
         IAC_CUDA(cudaGetLastError());
-        iac_status st = launch_frame_sums(ctx->sm_count, d_frames, npix, nframes, d_mask, threshold, step, nullptr,
-                                          d_mean_intensity, nullptr, ctx->d_counters, s);
+        iac_status st = launch_frame_sums(ctx, d_frames, npix, nframes, d_mask, threshold, step, nullptr,
+                                          d_mean_intensity, nullptr, s);
         if (st != IAC_OK) return st;
-        IAC_LAUNCHED(ctx);
     }
     return IAC_OK;
 }

@@ -84,3 +84,50 @@ def test_average_frames_many_frames(ctx, oracle_lib, rng, nframes, npix, thr, st
     else:
         np.testing.assert_array_equal(d_sum.cpu().numpy(), sum_o)
     assert ctx.check() == 0
+
+
+@pytest.mark.parametrize("npix", [8192, 16384 + 3, 5 * 4096 + 4, 40000])
+@pytest.mark.parametrize("nframes", [7, 300])
+@pytest.mark.parametrize("kind", ["positive", "noise", "negative", "ties", "whole numbers", "tiny and huge",
+                                  "powers of two", "zeros", "not finite"])
+def test_sequential_sums_in_any_order(ctx, oracle_lib, rng, npix, nframes, kind):
+    """The sequential FP32 sums that are formed as integer sums: sums that hover
+    around zero, that fall, that meet ties all the time or change their binade at
+    every pixel, that stay at a power of two, and that leave the finite numbers."""
+    import torch
+    o = oracle_lib
+    x = rng.gamma(0.6, 1.3, (nframes, npix)).astype(np.float32)
+    if kind == "noise":
+        x = rng.normal(0.0, 0.1, (nframes, npix)).astype(np.float32)
+    elif kind == "negative":
+        x = -x
+    elif kind == "ties":
+        x = (rng.integers(0, 9, (nframes, npix)) * 0.125 + 2.0 ** 20).astype(np.float32)
+    elif kind == "whole numbers":
+        x = rng.integers(0, 1 << 14, (nframes, npix)).astype(np.float32)
+    elif kind == "tiny and huge":
+        x = np.ldexp(x, rng.integers(-60, 30, (nframes, npix))).astype(np.float32)
+    elif kind == "powers of two":
+        x = np.zeros((nframes, npix), np.float32)
+        x[:, 5] = 1024.0
+        x[:, 6000:] = np.where(rng.random((nframes, npix - 6000)) < 0.5, 3e-5, -3e-5).astype(np.float32)
+    elif kind == "zeros":
+        x[:] = 0.0
+        x[1::2, -3] = 0.7
+    elif kind == "not finite":
+        x[0, npix // 2] = np.inf
+        x[1, npix // 3] = np.nan
+        x[2, 5] = -np.inf
+        x[3, npix - 1] = np.inf
+        x[4, [17, npix - 9]] = [np.inf, -np.inf]
+        x[5] *= np.float32(1e34)
+    mean_o, ph_o = np.zeros(nframes, np.float32), np.zeros(nframes, np.float32)
+    sum_o, discr_o = np.zeros(npix, np.float32), np.zeros(npix, np.int64)
+    with np.errstate(all="ignore"):
+        o.lib().iaco_average_frames(o.p(x), npix, nframes, None, -1e30, 0.0, o.p(sum_o), o.p(discr_o), o.p(mean_o),
+                                    o.p(ph_o))
+    d_sum = torch.zeros(npix, dtype=torch.float32, device="cuda")
+    d_mean = torch.zeros(nframes, dtype=torch.float32, device="cuda")
+    ctx.average_frames(torch.from_numpy(x).cuda(), npix, nframes, None, -1e30, 0.0, d_sum, None, d_mean)
+    np.testing.assert_array_equal(d_mean.cpu().numpy(), mean_o)
+    assert ctx.check() == 0
