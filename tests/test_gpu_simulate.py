@@ -227,3 +227,30 @@ def test_sparsify_matches_create_sparse_hit_list(ctx, oracle_lib):
             n = o.lib().iaco_sparse_hitlist(o.p(Im), o.p(km), npix, thr, step, 1, o.p(out))
             assert off[f + 1] - off[f] == n
             np.testing.assert_array_equal(ph[off[f]:off[f + 1]], out[:n])
+
+
+@pytest.mark.parametrize("npix", [1, 255, 2047, 2049, 9999])
+@pytest.mark.parametrize("mean", [0.001, 0.02, 0.6, 0.99999, 3.0, 60.0])
+def test_poisson_draws_by_mean(ctx, oracle_lib, npix, mean):
+    """The draws that are decided without the exponential and those that are not:
+    images of one mean, with pixels of intensity 0 and a bright one, against the
+    oracle's draws (its search is the same function; exp, log and cos in double)."""
+    import torch
+    from incohautocorrelate_b200 import capi
+    rng = np.random.default_rng(11)
+    nframes = 3
+    I = rng.gamma(0.5, 1.0, (nframes, npix)).astype(np.float32)
+    I[:, ::7] = 0.0
+    I[:, npix // 2] = 3.0
+    d = _dev(I)
+    ctx.simulate_photons(d, npix, nframes, 7, capi.PhotonParams(mean * npix, 1, 0.0, 2.0), 1234)
+    got = d.cpu().numpy()
+    mism = 0
+    for f in range(nframes):
+        factor = np.float32(mean * npix / float(I[f].astype(np.float64).sum()))
+        lam = (I[f] * factor).astype(np.float32)
+        want = np.zeros(npix, np.float32)
+        oracle_lib.lib().iaco_poisson_array(oracle_lib.p(lam), npix, 1234, RNG_POISSON | (7 + f), oracle_lib.p(want))
+        mism += int((2.0 * want != got[f]).sum())
+        assert (got[f][lam == 0.0] == 0.0).all()
+    assert mism <= 4
