@@ -13,7 +13,7 @@
 //                            by the isotropy, angle uniform), the rotated atom
 //                            positions, per-mode fluorescence roll and phases;
 //                            the event matrix is the inverse rotation.
-//  simulate_kernel           one thread per pixel, grid over (pixels, frames):
+//  simulate_kernel           two pixels per thread, grid over (pixels, frames):
 //                            per mode and sub-pixel, Psi = sum_j exp(i(k.r_j +
 //                            phi_j)) with the phase argument formed in FP32 in
 //                            the reference's order, then |Psi| (reference) or
@@ -48,16 +48,12 @@ constexpr float TWO_PI_HI = (float)TWO_PI_D;
 constexpr float TWO_PI_LO = (float)(TWO_PI_D - (double)TWO_PI_HI);
 constexpr float INV_TWO_PI = (float)(1.0 / TWO_PI_D);
 
-// the whole number of turns in a phase, rintf(arg / 2 pi) with ties to even, by
-// two FP32 adds on the FMA pipe: x + 1.5 * 2^23 rounds x to an integer in the
-// float's last place for |x| < 2^22 (phases below 2.6e7 rad; past that an FP32
+// The whole number of turns in a phase, rintf(arg / 2 pi) with ties to even, is
+// formed by two FP32 adds on the FMA pipe: x + 1.5 * 2^23 rounds x to an integer in
+// the float's last place for |x| < 2^22 (phases below 2.6e7 rad; past that an FP32
 // phase has lost every fraction of a turn anyway).  rintf is a conversion-unit
 // instruction, and that unit also runs the two MUFU operations of every term,
 // which bound the simulator.
-__device__ __forceinline__ float phase_turns(float arg)
-{
-    return fsub(fadd(fmul(arg, INV_TWO_PI), ROUND_MAGIC), ROUND_MAGIC);
-}
 
 struct CrystalArgs {
     const double *__restrict__ atoms;  // 3 doubles per atom
@@ -201,157 +197,102 @@ struct SimArgs {
     float wavelength;
     int amplitude_sq;  // 0: |Psi| as the reference, 1: |Psi|^2
     int accurate;      // 1: sincosf instead of explicit reduction + SFU
+    float neg_zero;    // -0.0f: fma(x, y, -0) is x * y rounded once, and never merges with an add
     float *__restrict__ out;  // [frame][pixel]
 };
 
 constexpr int SIM_THREADS = 128;
-constexpr int SIM_MAX_EM = 1024;  // emitters per (frame, mode) staged in shared memory
+constexpr int SIM_MAX_EM = 1024;  // emitters staged in shared memory at a time
 
-// pixels per thread of simulate_kernel: pixels p and p + SIM_THREADS share
-// every emitter load and the loop overhead; each pixel's sums keep their order
-constexpr int SIM_PIX = 2;
-
+// Two pixels per thread, p and p + SIM_THREADS: every FP32 operation of a term is
+// one f32x2 instruction for both (same roundings as two scalar ones), with the
+// emitter staged as pairs (x, x, y, y), (z, z, phase, phase).  Bound by the two
+// MUFU operations of a term: 5 x 5 x 8 emitters, 4 modes, 100 frames of 512^2
+// 10.8 ms = 0.83 of the SFU rate; with scalar FP32, whose issue slots ran
+// out beside the MUFU's, 11.7 ms (0.77).  An emitter list is staged once per mode;
+// one longer than SIM_MAX_EM streams through the stage in chunks, in order, for
+// every sub-pixel, so each pixel's sums always add the same terms in the same order.
+template <bool ACCURATE>
 __global__ void __launch_bounds__(SIM_THREADS) simulate_kernel(const SimArgs a)
 {
-    extern __shared__ float4 s_em[];  // [mode][SIM_MAX_EM window]
+    extern __shared__ float4 s_em[];  // two per emitter
     const uint32_t f = blockIdx.y;
-    const uint64_t p0 = blockIdx.x * (uint64_t)(SIM_PIX * SIM_THREADS) + threadIdx.x;
-    const uint32_t ncap = min(a.natoms, (uint32_t)SIM_MAX_EM);
-    for (uint32_t m = 0; m < a.nmodes; m++) {
-        const uint32_t n = min(a.em_count[(size_t)f * a.nmodes + m], ncap);
-        const float4 *src = a.em + ((size_t)f * a.nmodes + m) * a.natoms;
-        for (uint32_t i = threadIdx.x; i < n; i += SIM_THREADS) s_em[m * ncap + i] = src[i];
-    }
-    __syncthreads();
-    if (p0 >= a.npix) return;
-    uint64_t px[SIM_PIX];
-    float pc[SIM_PIX][3];
-#pragma unroll
-    for (int q = 0; q < SIM_PIX; q++) {
-        px[q] = p0 + (uint64_t)q * SIM_THREADS;
-        const uint64_t pp = px[q] < a.npix ? px[q] : p0;  // a pixel past the end repeats p0, unwritten
-#pragma unroll
-        for (int d = 0; d < 3; d++) pc[q][d] = a.pm[3 * pp + d];
-    }
+    const uint64_t p0 = blockIdx.x * (uint64_t)(2 * SIM_THREADS) + threadIdx.x, p1 = p0 + SIM_THREADS;
+    // a pixel past the end repeats the first, unwritten
+    const float *pc0 = a.pm + 3 * (p0 < a.npix ? p0 : 0), *pc1 = a.pm + 3 * (p1 < a.npix ? p1 : 0);
+    const float2 c0 = make_float2(pc0[0], pc1[0]), c1 = make_float2(pc0[1], pc1[1]), c2 = make_float2(pc0[2], pc1[2]);
+    const float2 nz = make_float2(a.neg_zero, a.neg_zero);
+    auto mul = [&](float2 x, float2 y) { return f2fma(x, y, nz); };
+    auto dup = [](float x) { return make_float2(x, x); };
     const float nsub = (float)((2 * a.susa + 1) * (2 * a.susa + 1));
-    float total[SIM_PIX];
-#pragma unroll
-    for (int q = 0; q < SIM_PIX; q++) total[q] = 0.0f;
-    for (uint32_t m = 0; m < a.nmodes; m++) {
-        const uint32_t n = min(a.em_count[(size_t)f * a.nmodes + m], ncap);
-        const float4 *E = s_em + m * ncap;
-        float acc[SIM_PIX];
-#pragma unroll
-        for (int q = 0; q < SIM_PIX; q++) acc[q] = 0.0f;
-        for (int v = -a.susa; v <= a.susa; v++)
-            for (int u = -a.susa; u <= a.susa; u++) {
-                float k[SIM_PIX][3], re[SIM_PIX], im[SIM_PIX];
-#pragma unroll
-                for (int q = 0; q < SIM_PIX; q++) {
-                    // IAC/kernel.cl:823-832
-                    const float c0 = fadd(fadd(pc[q][0], fmul((float)v, a.vs[0])), fmul((float)u, a.us[0]));
-                    const float c1 = fadd(fadd(pc[q][1], fmul((float)v, a.vs[1])), fmul((float)u, a.us[1]));
-                    const float c2 = fadd(fadd(pc[q][2], fmul((float)v, a.vs[2])), fmul((float)u, a.us[2]));
-                    float nk = (float)(1.0 / (double)norm3(c0, c1, c2));
-                    nk = (float)((double)nk * ((2.0 * 3.1415926535897932) / (double)a.wavelength));
-                    k[q][0] = fmul(c0, nk);
-                    k[q][1] = fmul(c1, nk);
-                    k[q][2] = fmul(c2, nk);
-                    re[q] = 0.0f;
-                    im[q] = 0.0f;
-                }
-                for (uint32_t i = 0; i < n; i++) {
-                    const float4 e = E[i];
-#pragma unroll
-                    for (int q = 0; q < SIM_PIX; q++) {
-                        float arg = fmul(k[q][0], e.x);
-                        arg = fadd(arg, fmul(k[q][1], e.y));
-                        arg = fadd(arg, fmul(k[q][2], e.z));
-                        arg = fadd(arg, e.w);
-                        float sn, cs;
-                        if (a.accurate) {
-                            sincosf(arg, &sn, &cs);
-                        } else {
-                            const float kk = phase_turns(arg);
-                            const float r = fmaf(-kk, TWO_PI_LO, fmaf(-kk, TWO_PI_HI, arg));
-                            __sincosf(r, &sn, &cs);
-                        }
-                        re[q] = fadd(re[q], cs);
-                        im[q] = fadd(im[q], sn);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < SIM_PIX; q++) {
-                    const float a2 = fadd(fmul(re[q], re[q]), fmul(im[q], im[q]));
-                    acc[q] = fadd(acc[q], a.amplitude_sq ? a2 : __fsqrt_rn(a2));
-                }
-            }
-#pragma unroll
-        for (int q = 0; q < SIM_PIX; q++) total[q] = fadd(total[q], __fdiv_rn(acc[q], nsub));  // as ParAdd sums modes
-    }
-#pragma unroll
-    for (int q = 0; q < SIM_PIX; q++)
-        if (px[q] < a.npix) a.out[(size_t)f * a.npix + px[q]] = total[q];
-}
-
-// simulate_kernel for crystals whose emitters do not fit the shared-memory
-// stage (more than SIM_MAX_EM, or modes x emitters past 200 KB): per mode and
-// sub-pixel the emitters stream through a stage of SIM_MAX_EM, chunk by chunk
-// in emitter order, so every pixel's phase sum adds the same terms in the same
-// order as the staged kernel
-__global__ void __launch_bounds__(SIM_THREADS) simulate_chunked_kernel(const SimArgs a)
-{
-    __shared__ float4 s_em[SIM_MAX_EM];
-    const uint32_t f = blockIdx.y;
-    const uint64_t p = blockIdx.x * (uint64_t)SIM_THREADS + threadIdx.x;
-    const bool live = p < a.npix;
-    const float pc0 = live ? a.pm[3 * p] : 0.0f, pc1 = live ? a.pm[3 * p + 1] : 0.0f,
-                pc2 = live ? a.pm[3 * p + 2] : 0.0f;
-    const float nsub = (float)((2 * a.susa + 1) * (2 * a.susa + 1));
-    float total = 0.0f;
+    float total0 = 0.0f, total1 = 0.0f;
     for (uint32_t m = 0; m < a.nmodes; m++) {
         const uint32_t n = min(a.em_count[(size_t)f * a.nmodes + m], a.natoms);
         const float4 *src = a.em + ((size_t)f * a.nmodes + m) * a.natoms;
-        float acc = 0.0f;
+        float acc0 = 0.0f, acc1 = 0.0f;
+        bool staged = false;
         for (int v = -a.susa; v <= a.susa; v++)
             for (int u = -a.susa; u <= a.susa; u++) {
-                const float c0 = fadd(fadd(pc0, fmul((float)v, a.vs[0])), fmul((float)u, a.us[0]));
-                const float c1 = fadd(fadd(pc1, fmul((float)v, a.vs[1])), fmul((float)u, a.us[1]));
-                const float c2 = fadd(fadd(pc2, fmul((float)v, a.vs[2])), fmul((float)u, a.us[2]));
-                float nk = live ? (float)(1.0 / (double)norm3(c0, c1, c2)) : 0.0f;
-                nk = (float)((double)nk * ((2.0 * 3.1415926535897932) / (double)a.wavelength));
-                const float k0 = fmul(c0, nk), k1 = fmul(c1, nk), k2 = fmul(c2, nk);
-                float re = 0.0f, im = 0.0f;
+                // IAC/kernel.cl:823-832
+                auto wave = [&](float x, float y, float z, float k[3]) {
+                    x = fadd(fadd(x, fmul((float)v, a.vs[0])), fmul((float)u, a.us[0]));
+                    y = fadd(fadd(y, fmul((float)v, a.vs[1])), fmul((float)u, a.us[1]));
+                    z = fadd(fadd(z, fmul((float)v, a.vs[2])), fmul((float)u, a.us[2]));
+                    float nk = (float)(1.0 / (double)norm3(x, y, z));
+                    nk = (float)((double)nk * ((2.0 * 3.1415926535897932) / (double)a.wavelength));
+                    k[0] = fmul(x, nk);
+                    k[1] = fmul(y, nk);
+                    k[2] = fmul(z, nk);
+                };
+                float ka[3], kb[3];
+                wave(c0.x, c1.x, c2.x, ka);
+                wave(c0.y, c1.y, c2.y, kb);
+                const float2 k0 = make_float2(ka[0], kb[0]), k1 = make_float2(ka[1], kb[1]), k2 = make_float2(ka[2], kb[2]);
+                float2 re = make_float2(0.0f, 0.0f), im = re;
                 for (uint32_t c = 0; c < n; c += SIM_MAX_EM) {
                     const uint32_t cn = min(n - c, (uint32_t)SIM_MAX_EM);
-                    __syncthreads();  // the previous chunk is read
-                    for (uint32_t i = threadIdx.x; i < cn; i += SIM_THREADS) s_em[i] = src[c + i];
-                    __syncthreads();
-                    if (!live) continue;
-                    for (uint32_t i = 0; i < cn; i++) {
-                        const float4 e = s_em[i];
-                        float arg = fmul(k0, e.x);
-                        arg = fadd(arg, fmul(k1, e.y));
-                        arg = fadd(arg, fmul(k2, e.z));
-                        arg = fadd(arg, e.w);
-                        float sn, cs;
-                        if (a.accurate) {
-                            sincosf(arg, &sn, &cs);
-                        } else {
-                            const float kk = phase_turns(arg);
-                            const float r = fmaf(-kk, TWO_PI_LO, fmaf(-kk, TWO_PI_HI, arg));
-                            __sincosf(r, &sn, &cs);
+                    if (!staged) {
+                        __syncthreads();  // the last stage is read
+                        for (uint32_t i = threadIdx.x; i < cn; i += SIM_THREADS) {
+                            const float4 e = src[c + i];
+                            s_em[2 * i] = make_float4(e.x, e.x, e.y, e.y);
+                            s_em[2 * i + 1] = make_float4(e.z, e.z, e.w, e.w);
                         }
-                        re = fadd(re, cs);
-                        im = fadd(im, sn);
+                        __syncthreads();
+                        staged = n <= (uint32_t)SIM_MAX_EM;
+                    }
+#pragma unroll 4
+                    for (uint32_t i = 0; i < cn; i++) {
+                        const float4 ea = s_em[2 * i], eb = s_em[2 * i + 1];
+                        float2 arg = mul(k0, make_float2(ea.x, ea.y));
+                        arg = f2add(arg, mul(k1, make_float2(ea.z, ea.w)));
+                        arg = f2add(arg, mul(k2, make_float2(eb.x, eb.y)));
+                        arg = f2add(arg, make_float2(eb.z, eb.w));
+                        float2 sn, cs;
+                        if (ACCURATE) {
+                            sincosf(arg.x, &sn.x, &cs.x);
+                            sincosf(arg.y, &sn.y, &cs.y);
+                        } else {
+                            // the whole turns of the phase by two adds
+                            const float2 t = f2sub(f2add(mul(arg, dup(INV_TWO_PI)), dup(ROUND_MAGIC)), dup(ROUND_MAGIC));
+                            const float2 nt = make_float2(-t.x, -t.y);
+                            const float2 r = f2fma(nt, dup(TWO_PI_LO), f2fma(nt, dup(TWO_PI_HI), arg));
+                            __sincosf(r.x, &sn.x, &cs.x);
+                            __sincosf(r.y, &sn.y, &cs.y);
+                        }
+                        re = f2add(re, cs);
+                        im = f2add(im, sn);
                     }
                 }
-                const float a2 = fadd(fmul(re, re), fmul(im, im));
-                acc = fadd(acc, a.amplitude_sq ? a2 : __fsqrt_rn(a2));
+                const float q0 = fadd(fmul(re.x, re.x), fmul(im.x, im.x)), q1 = fadd(fmul(re.y, re.y), fmul(im.y, im.y));
+                acc0 = fadd(acc0, a.amplitude_sq ? q0 : __fsqrt_rn(q0));
+                acc1 = fadd(acc1, a.amplitude_sq ? q1 : __fsqrt_rn(q1));
             }
-        total = fadd(total, __fdiv_rn(acc, nsub));
+        total0 = fadd(total0, __fdiv_rn(acc0, nsub));  // as ParAdd sums modes
+        total1 = fadd(total1, __fdiv_rn(acc1, nsub));
     }
-    if (live) a.out[(size_t)f * a.npix + p] = total;
+    if (p0 < a.npix) a.out[(size_t)f * a.npix + p0] = total0;
+    if (p1 < a.npix) a.out[(size_t)f * a.npix + p1] = total1;
 }
 
 // per-frame double sum, one CTA per frame: SUM_THREADS chains of adds, each over
@@ -775,16 +716,13 @@ iac_status iac_simulate_intensity(iac_ctx *ctx, const float *d_pixel_map, uint64
     a.amplitude_sq = sp->intensity_squared;
     a.accurate = sp->accurate_sincos;
     a.out = d_intensity;
-    dim3 grid((unsigned)((npix + SIM_THREADS - 1) / SIM_THREADS), nframes);
-    if (natoms <= (uint32_t)SIM_MAX_EM && (uint64_t)nmodes * natoms * 16 <= 200 * 1024) {
-        // every mode's emitters staged at once
-        const size_t smem = sizeof(float4) * nmodes * natoms;
-        IAC_CUDA(cudaFuncSetAttribute(simulate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const dim3 grid2((unsigned)((npix + SIM_PIX * SIM_THREADS - 1) / (SIM_PIX * SIM_THREADS)), nframes);
-        simulate_kernel<<<grid2, SIM_THREADS, smem, as_stream(stream)>>>(a);
-    } else {
-        simulate_chunked_kernel<<<grid, SIM_THREADS, 0, as_stream(stream)>>>(a);
-    }
+    a.neg_zero = -0.0f;
+    const dim3 grid((unsigned)((npix + 2 * SIM_THREADS - 1) / (2 * SIM_THREADS)), nframes);
+    const size_t smem = 2 * sizeof(float4) * std::min<uint32_t>(natoms, SIM_MAX_EM);
+    if (a.accurate)
+        simulate_kernel<true><<<grid, SIM_THREADS, smem, as_stream(stream)>>>(a);
+    else
+        simulate_kernel<false><<<grid, SIM_THREADS, smem, as_stream(stream)>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
     return IAC_OK;

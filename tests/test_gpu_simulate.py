@@ -254,3 +254,40 @@ def test_poisson_draws_by_mean(ctx, oracle_lib, npix, mean):
         mism += int((2.0 * want != got[f]).sum())
         assert (got[f][lam == 0.0] == 0.0).all()
     assert mism <= 4
+
+
+@pytest.mark.parametrize("npix", [1, 127, 129, 257])
+@pytest.mark.parametrize("natoms", [1, 5, 1023, 1024, 1025, 2049])
+@pytest.mark.parametrize("susa,accurate", [(0, 0), (1, 0), (0, 1)])
+def test_intensity_at_the_edges_of_the_stage(ctx, oracle_lib, npix, natoms, susa, accurate):
+    """Odd pixel counts (the second pixel of a thread absent), emitter lists at the
+    edges of the shared-memory stage and modes of different length: the tolerance
+    of the test above against the oracle."""
+    import torch
+    from incohautocorrelate_b200 import capi
+    o = oracle_lib
+    rng = np.random.default_rng(13)
+    pm = np.ascontiguousarray(_sim_setup(o, npx=17)[: 3 * npix])
+    nmodes, nframes, us = 2, 2, 2e7 / (2 * susa + 1)
+    em = np.concatenate([rng.uniform(-15, 15, (nframes, nmodes, natoms, 3)),
+                         rng.uniform(0, 2 * np.pi, (nframes, nmodes, natoms, 1))], 3).astype(np.float32)
+    cnt = np.full((nframes, nmodes), natoms, np.int32)
+    cnt[1, 0] = (natoms + 1) // 2
+    sp = capi.SimParams(susa, (C.c_double * 3)(us, 0, 0), (C.c_double * 3)(0, us, 0), 1.55, 1, accurate)
+    out = torch.zeros((nframes, npix), dtype=torch.float32, device="cuda")
+    ctx.simulate_intensity(_dev(pm), npix, _dev(em), _dev(cnt), natoms, nmodes, nframes, sp, out)
+    got = out.cpu().numpy()
+    for f in range(nframes):
+        want = np.zeros(npix, np.float32)
+        peak = 0.0
+        for m in range(nmodes):
+            n = int(cnt[f, m])
+            e = np.ascontiguousarray(em[f, m, :n])
+            P = np.array([n, 1, susa, us, 0, 0, 0, us, 0, 1.55], np.float64)
+            t = np.zeros(npix, np.float32)
+            o.lib().iaco_simulate_crystal(o.p(pm), npix, o.p(e), n, o.p(P), 1, o.p(t))
+            want += t
+            peak += float(n)
+        # |Psi|^2 of n terms: each term's error of about 1e-6 rad adds to an amplitude of about sqrt(n)
+        np.testing.assert_allclose(got[f], want, atol=2e-5 * max(float(want.max()), peak), rtol=0)
+    assert ctx.check() == 0
