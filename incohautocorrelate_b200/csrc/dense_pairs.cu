@@ -45,7 +45,7 @@ constexpr int WINDOW_WORDS = 2048;  // shared-memory window: 2048 split 64-bit c
 struct DenseArgs {
     const float *__restrict__ I;
     const float *__restrict__ K;     // 3 floats per pixel
-    const float4 *__restrict__ box;  // per tile: min (x,y,z), max (x,y,z) as 2 float4
+    const float4 *__restrict__ box;  // per tile: min (x,y,z), max |I|; max (x,y,z), min I
     unsigned long long *__restrict__ out;
     unsigned long long *queue;
     DeviceCounters *counters;
@@ -59,6 +59,8 @@ struct DenseArgs {
     float maxq, maxq2;
     float vpdq;
     double mult;
+    float mult_f;    // Multiplicator as a float when that is exact (and an integer), else 0
+    float neg_zero;  // -0.0f: fma(x, y, -0) is x * y rounded once, and never merges with an add
     // C(q) small mesh
     int ab, sc, cab, cc;  // sizes and centres
     int ka, kb, kc;       // q axis on mesh fs / ms / ss
@@ -119,12 +121,19 @@ __global__ void tile_box_kernel(const DenseArgs a, float4 *__restrict__ box)
     const float *__restrict__ K = a.K;
     const float *__restrict__ I = a.I;
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float imax = 0.0f;  // largest |I| of the tile (NaN propagates: the tile then takes no fast path)
+    // largest |I| of the tile (infinite for a NaN or a k-vector that is not finite: the
+    // tile then takes no fast path) and smallest I
+    float imax = 0.0f, imin = 0.0f;
     if (i < a.npix && I[i] != 0.0f) {  // zero-intensity pixels never contribute
+        bool finite = true;
 #pragma unroll
-        for (int d = 0; d < 3; d++) mn[d] = mx[d] = K[3 * i + d];
+        for (int d = 0; d < 3; d++) {
+            mn[d] = mx[d] = K[3 * i + d];
+            finite = finite && fabsf(mn[d]) < INFINITY;
+        }
         imax = fabsf(I[i]);
-        if (imax != imax) imax = INFINITY;
+        imin = I[i];
+        if (imax != imax || !finite) imax = INFINITY;
     }
 #pragma unroll
     for (int d = 0; d < 3; d++)
@@ -132,8 +141,11 @@ __global__ void tile_box_kernel(const DenseArgs a, float4 *__restrict__ box)
             mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
             mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
         }
-    for (int o = 16; o; o >>= 1) imax = fmaxf(imax, __shfl_xor_sync(0xffffffffu, imax, o));
-    __shared__ float s[7][DTILE / 32];
+    for (int o = 16; o; o >>= 1) {
+        imax = fmaxf(imax, __shfl_xor_sync(0xffffffffu, imax, o));
+        imin = fminf(imin, __shfl_xor_sync(0xffffffffu, imin, o));
+    }
+    __shared__ float s[8][DTILE / 32];
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
         for (int d = 0; d < 3; d++) {
@@ -141,16 +153,17 @@ __global__ void tile_box_kernel(const DenseArgs a, float4 *__restrict__ box)
             s[3 + d][w] = mx[d];
         }
         s[6][w] = imax;
+        s[7][w] = imin;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        float r[7];
-        for (int d = 0; d < 7; d++) {
+        float r[8];
+        for (int d = 0; d < 8; d++) {
             r[d] = s[d][0];
-            for (int j = 1; j < DTILE / 32; j++) r[d] = d < 3 ? fminf(r[d], s[d][j]) : fmaxf(r[d], s[d][j]);
+            for (int j = 1; j < DTILE / 32; j++) r[d] = d < 3 || d == 7 ? fminf(r[d], s[d][j]) : fmaxf(r[d], s[d][j]);
         }
         box[2 * t] = make_float4(r[0], r[1], r[2], r[6]);
-        box[2 * t + 1] = make_float4(r[3], r[4], r[5], 0.f);
+        box[2 * t + 1] = make_float4(r[3], r[4], r[5], r[7]);
     }
 }
 
@@ -479,6 +492,161 @@ __device__ __forceinline__ void cq_pairs_win2(const DenseArgs &a, const Window &
     if (acc) shared_add_u64_split(win, win + WINDOW_WORDS, (uint32_t)cur, acc);
 }
 
+// ---------------------------------------------------------------------------
+// Tiles whose intensities are not negative and whose products times the
+// Multiplicator stay below SMALL_VALUE (2^23), which the usual maps do (the
+// Multiplicator puts the mean product between 1e5 and 1e6): the values need no
+// 64-bit arithmetic.  For an integer Multiplicator M below 2^24, p M + 2^23 rounded
+// toward zero is 2^23 + floor(p M), one f32x2 fma for two pairs.  A run of 256
+// pairs sums to less than 2^31 and goes to the window in two halves, its low 16
+// bits into one word and the rest into another: a tile pair adds at most 65 536
+// runs, so neither word overflows and no add has to return anything.  Pixels of
+// intensity 0 (masked, or absent from a ragged tile) are staged at a corner of
+// the tile's box, so every pair lands in the window and their value of 0 adds
+// nothing.  1024 x 512 map, 199-edge mesh, nearest: 214.9 -> 147.4 ms (39 instructions a
+// pair, issue 85 %, shared-memory wavefronts 74 % of peak); linear at 244 x 250, 127-edge
+// mesh: 17.6 -> 8.5 ms.  Larger products keep the 64-bit paths above.
+// ---------------------------------------------------------------------------
+constexpr float SMALL_VALUE = 8388608.0f;
+
+__device__ __forceinline__ bool small_values(const DenseArgs &a, const float4 p0, const float4 p1, const float4 q0,
+                                             const float4 q1)
+{
+    // a Multiplicator past 1e30 could lift products that the 1e-37 cut drops to whole numbers
+    return a.mult > 0.0 && a.mult < 1e30 && p1.w >= 0.0f && q1.w >= 0.0f &&
+           __fmul_ru(__fmul_ru(p0.w, q0.w), __double2float_ru(a.mult)) < SMALL_VALUE;
+}
+
+// add `acc` (< 2^31) in two halves at window word `at` if `on`
+__device__ __forceinline__ void window_add_halves(uint32_t win, int at, uint32_t acc, bool on)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p red.shared.add.u32 [%1], %2;\n\t"
+        "@p red.shared.add.u32 [%1+%4], %3;\n\t}" ::"r"((int)on),
+        "r"(win + 4u * (uint32_t)at), "r"(acc & 0xffffu), "r"(acc >> 16), "n"(4 * WINDOW_WORDS)
+        : "memory");
+}
+
+// nearest voxel, two staged pixels per step; win: shared-memory address of the window
+template <int KA, int KB, int KC, bool CHECK>
+__device__ __forceinline__ void cq_pairs_small(const DenseArgs &a, const Window &w, uint32_t win, const float4 *sp, int j0,
+                                               float k0, float k1, float k2, float Ia)
+{
+    const int D0 = w.dim[0], D01 = w.dim[0] * w.dim[1];
+    const int base = (a.cab - w.lo[0]) + D0 * (a.cab - w.lo[1]) + D01 * (a.cc - w.lo[2]);
+    auto dup = [](float x) { return make_float2(x, x); };
+    int cur = 0;  // pending run: window word, sum (0 before the first pair)
+    uint32_t acc = 0;
+    auto put = [&](int key, uint32_t v) {
+        const bool brk = key != cur;
+        window_add_halves(win, cur, acc, brk);
+        acc = (brk ? 0u : acc) + v;
+        cur = key;
+    };
+    auto step = [&](int jp, bool lo_on) {
+        const float4 A = sp[2 * jp], B = sp[2 * jp + 1];
+        const float2 pv = f2mul(dup(Ia), make_float2(B.z, B.w));
+        float2 qx = f2sub(dup(k0), make_float2(A.x, A.y)), qy = f2sub(dup(k1), make_float2(A.z, A.w)),
+               qz = f2sub(dup(k2), make_float2(B.x, B.y));
+        const float2 vb = f2fma_rz(pv, dup(a.mult_f), dup(8388608.0f));
+        uint32_t v0 = __float_as_uint(vb.x) - 0x4B000000u, v1 = __float_as_uint(vb.y) - 0x4B000000u;
+        bool ok0 = lo_on, ok1 = true;
+        if (CHECK) {
+            const float2 nz = dup(a.neg_zero);
+            const float2 s = f2add(f2add(f2fma(qx, qx, nz), f2fma(qy, qy, nz)), f2fma(qz, qz, nz));
+            ok0 = ok0 && s.x <= a.maxq2;
+            ok1 = s.y <= a.maxq2;
+        }
+        const float2 vp = dup(a.vpdq);
+        qx = f2mul(qx, vp);
+        qy = f2mul(qy, vp);
+        qz = f2mul(qz, vp);
+        const int2 f = f2round_half_away(KA == 0 ? qx : KA == 1 ? qy : qz);
+        const int2 m = f2round_half_away(KB == 0 ? qx : KB == 1 ? qy : qz);
+        const int2 sz = f2round_half_away(KC == 0 ? qx : KC == 1 ? qy : qz);
+        // a pair that is off adds 0 to the pending run
+        const int key0 = base + f.x + D0 * m.x + D01 * sz.x, key1 = base + f.y + D0 * m.y + D01 * sz.y;
+        if (CHECK || !lo_on)
+            put(ok0 ? key0 : cur, ok0 ? v0 : 0u);
+        else
+            put(key0, v0);
+        if (CHECK)
+            put(ok1 ? key1 : cur, ok1 ? v1 : 0u);
+        else
+            put(key1, v1);
+    };
+    int jp = j0 >> 1;
+    if (j0 & 1) step(jp++, false);
+#pragma unroll 2
+    for (; jp < DTILE / 2; jp++) step(jp, true);
+    window_add_halves(win, cur, acc, true);
+}
+
+// 8-corner linear, for the same tiles and any Multiplicator: the floor of a
+// corner's double product is the low word of that product plus 2^52 rounded toward
+// zero, and the eight sums of a run are 32-bit words, which go to the window's
+// split counters with their carries.
+template <int KA, int KB, int KC, bool CHECK>
+__device__ __forceinline__ void cq_pairs_small_linear(const DenseArgs &a, const Window &w, uint32_t win, const float4 *sq,
+                                                      int j0, float k0, float k1, float k2, float Ia)
+{
+    const int D0 = w.dim[0], D01 = w.dim[0] * w.dim[1];
+    const int base = (a.cab - w.lo[0]) + D0 * (a.cab - w.lo[1]) + D01 * (a.cc - w.lo[2]);
+    int cur = 0;
+    uint32_t acc[8];  // [4 fs + 2 ms + ss]
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[c] = 0;
+    auto at = [&](int c) { return win + 4u * (uint32_t)(cur + (c >> 2) + ((c >> 1) & 1) * D0 + (c & 1) * D01); };
+    auto flush = [&]() {
+        uint32_t old[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old[c]) : "r"(at(c)), "r"(acc[c]) : "memory");
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            if (old[c] + acc[c] < old[c])  // rare: the carry out of the low word
+                asm volatile("red.shared.add.u32 [%0+%1], 1;" ::"r"(at(c)), "n"(4 * WINDOW_WORDS) : "memory");
+            acc[c] = 0;
+        }
+    };
+    // floor of |x| < 2^22 as an integer; frac: x - floor x, as the reference forms it
+    auto floor_frac = [](float x, float &frac) {
+        const float t = __fadd_rd(x, ROUND_MAGIC);
+        frac = fsub(x, fsub(t, ROUND_MAGIC));
+        return __float_as_int(t) - 0x4B400000;
+    };
+#pragma unroll 1
+    for (int j = j0; j < DTILE; j++) {
+        const float4 b = sq[j];
+        float pv = fmul(Ia, b.w);
+        float qx = fsub(k0, b.x), qy = fsub(k1, b.y), qz = fsub(k2, b.z);
+        const bool ok = !CHECK || fadd(fadd(fmul(qx, qx), fmul(qy, qy)), fmul(qz, qz)) <= a.maxq2;
+        qx = fmul(qx, a.vpdq);
+        qy = fmul(qy, a.vpdq);
+        qz = fmul(qz, a.vpdq);
+        float ff, fm, fz;
+        const int f = floor_frac(axis<KA>(qx, qy, qz, 0), ff), m = floor_frac(axis<KB>(qx, qy, qz, 0), fm),
+                  s = floor_frac(axis<KC>(qx, qy, qz, 0), fz);
+        const int key = ok ? base + f + D0 * m + D01 * s : cur;
+        if (key != cur) {
+            flush();
+            cur = key;
+        }
+        const double vm = dmul((double)(ok ? pv : 0.0f), a.mult);
+        // IAC/kernel.cl:139-179: Sep = 1 - (q - floor q) in float
+        const double sf = (double)fsub(1.0f, ff), sm = (double)fsub(1.0f, fm), sz = (double)fsub(1.0f, fz);
+        const double xf[2] = {sf, dsub(1.0, sf)}, yf[2] = {sm, dsub(1.0, sm)}, zf[2] = {sz, dsub(1.0, sz)};
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+            const double xy = dmul(xf[c >> 2], yf[(c >> 1) & 1]);
+#pragma unroll
+            for (int z = 0; z < 2; z++)
+                acc[c + z] += (uint32_t)__double2loint(__dadd_rz(dmul(vm, dmul(xy, zf[z])), 4503599627370496.0));
+        }
+    }
+    flush();
+}
+
 // upper bound of |k_a - k_b| over two boxes is below MaxQ with a margin that
 // covers the FP32 rounding of the per-pair test (every pair passes it)
 __device__ __forceinline__ bool boxes_within(const float4 a0, const float4 a1, const float4 b0, const float4 b1,
@@ -499,7 +667,7 @@ __device__ __forceinline__ int own_pixel(int t)
 }
 
 template <int INTERP, int KA, int KB, int KC>
-__global__ void __launch_bounds__(DTILE, 5) cq_small_kernel(const DenseArgs a)
+__global__ void __launch_bounds__(DTILE, INTERP ? 4 : 6) cq_small_kernel(const DenseArgs a)
 {
     __shared__ float4 sq[DTILE];
     __shared__ uint32_t win[2 * WINDOW_WORDS];  // split 64-bit counters: low words, then high words
@@ -540,14 +708,17 @@ __global__ void __launch_bounds__(DTILE, 5) cq_small_kernel(const DenseArgs a)
             if (w.on)
                 for (int i = threadIdx.x; i < words; i += DTILE) win[i] = win[WINDOW_WORDS + i] = 0u;
         }
+        const bool small = KA >= 0 && w.on && (INTERP || a.mult_f != 0.0f) && small_values(a, p0, p1, q0, q1);
         // integer Multiplicator and every product of the two tiles below 2^23
         // (the tiles' largest |I|): the packed window path
-        const bool packed = INTERP == 0 && KA >= 0 && w.on && a.mult_int != 0u && fmul(p0.w, q0.w) < 8388608.0f;
+        const bool packed =
+            INTERP == 0 && (small || (KA >= 0 && w.on && a.mult_int != 0u && fmul(p0.w, q0.w) < 8388608.0f));
         // stage tile Q: (k, I) per pixel, or interleaved per pixel pair for the packed path
         {
             const uint64_t j = tile_pixel(a, Q, threadIdx.x);
-            const float4 v = j < a.npix ? make_float4(a.K[3 * j], a.K[3 * j + 1], a.K[3 * j + 2], a.I[j])
-                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 v = j < a.npix ? make_float4(a.K[3 * j], a.K[3 * j + 1], a.K[3 * j + 2], a.I[j])
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (small && v.w == 0.0f) v = make_float4(q0.x, q0.y, q0.z, 0.f);  // adds 0 inside the window
             if (packed) {
                 float *spf = reinterpret_cast<float *>(sq) + (threadIdx.x >> 1) * 8 + (threadIdx.x & 1);
                 spf[0] = v.x;
@@ -575,7 +746,18 @@ __global__ void __launch_bounds__(DTILE, 5) cq_small_kernel(const DenseArgs a)
                     self = a.mult_int ? scaled_floor(sv, a.mult_int) : d2u64(dmul((double)sv, a.mult));
             }
             const int j0 = (P == Q) ? own + 1 : 0;
-            if (packed) {
+            if (small) {
+                const uint32_t wa = (uint32_t)__cvta_generic_to_shared(win);
+                if (Ia == 0.0f) {
+                } else if (INTERP && check)
+                    cq_pairs_small_linear<KA, KB, KC, true>(a, w, wa, sq, j0, k0, k1, k2, Ia);
+                else if (INTERP)
+                    cq_pairs_small_linear<KA, KB, KC, false>(a, w, wa, sq, j0, k0, k1, k2, Ia);
+                else if (check)
+                    cq_pairs_small<KA, KB, KC, true>(a, w, wa, sq, j0, k0, k1, k2, Ia);
+                else
+                    cq_pairs_small<KA, KB, KC, false>(a, w, wa, sq, j0, k0, k1, k2, Ia);
+            } else if (packed) {
                 if (check)
                     cq_pairs_win2<KA, KB, KC, true>(a, w, win, sq, j0, k0, k1, k2, Ia);
                 else
@@ -622,7 +804,9 @@ __global__ void __launch_bounds__(DTILE, 5) cq_small_kernel(const DenseArgs a)
         if (w.on) {
             const int words = w.dim[0] * w.dim[1] * w.dim[2];
             for (int i = threadIdx.x; i < words; i += DTILE) {
-                const unsigned long long v = split_word(win, win + WINDOW_WORDS, i);
+                const unsigned long long v =
+                    small && !INTERP ? win[i] + ((unsigned long long)win[WINDOW_WORDS + i] << 16)
+                                     : split_word(win, win + WINDOW_WORDS, i);
                 if (!v) continue;
                 const int x = i % w.dim[0], y = (i / w.dim[0]) % w.dim[1], z = i / (w.dim[0] * w.dim[1]);
                 global_put_pair(a, x + w.lo[0], y + w.lo[1], z + w.lo[2], v);
@@ -913,6 +1097,8 @@ static iac_status prepare(iac_ctx *ctx, void *stream, const float *d_I, const fl
         a.nx = a.ny = a.ptx = 0;
         a.ntiles = (uint32_t)((npix + DTILE - 1) / DTILE);
     }
+    a.mult_f = a.mult_int && (double)(float)mult == mult ? (float)mult : 0.0f;
+    a.neg_zero = -0.0f;
     a.npairs = (unsigned long long)a.ntiles * (a.ntiles + 1) / 2;
     a.part = 0;
     a.nparts = 1;

@@ -318,6 +318,15 @@ __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c)
     return r;
 }
 
+__device__ __forceinline__ float2 f2fma_rz(float2 a, float2 b, float2 c)  // rounded toward zero
+{
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rz.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
 // as a float; exact for |x| < 2^23 (callers bound x), NaN stays NaN
 __device__ __forceinline__ float round_away_rz_f(float x)
 {

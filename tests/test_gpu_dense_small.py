@@ -1,0 +1,55 @@
+"""Dense C(q) tiles whose values stay below 2^23 (their own kernels'
+path) next to tiles that leave it, bit for bit against the oracle: values at
+the limit, negative intensities, masked pixels whose k is far outside the mesh,
+MaxQ cuts, ragged tiles, Multiplicators that are no integers or no floats."""
+import numpy as np
+import pytest
+
+from helpers import small_detector, to_capi_shape
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _cases(rng, npix, km):
+    """(name, I, kmap, Multiplicator)"""
+    I = rng.uniform(0.05, 1.5, npix).astype(np.float32)
+    I[rng.random(npix) < 0.1] = 0
+    edge = I.copy()
+    top = float(edge.max())
+    limit = 2.0 ** 23 / top ** 2  # the tiles of the brightest pixel end just past the limit, others below
+    far = km.copy().reshape(-1, 3)
+    far[I == 0] = np.float32(1e18)
+    negative = I.copy()
+    negative[3::97] *= -1
+    dim = (I * np.float32(1e-18)).astype(np.float32)  # products around the 1e-37 cut
+    yield "limit", edge, km, float(np.floor(limit))
+    yield "past", edge, km, float(np.ceil(limit) + 1)
+    yield "fraction", I, km, 100000.5
+    yield "no float", I, km, 16777217.0
+    yield "far masked", I, far.reshape(-1), 123457.0
+    yield "negative", negative, km, 100000.0
+    yield "dim", dim, km, 2.0 ** 29 - 1
+    yield "huge", dim, km, 1e38
+    yield "all masked", np.zeros(npix, np.float32), km, 1000.0
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+@pytest.mark.parametrize("ny,nx,cut", [(16, 16, 1.0), (17, 31, 0.6), (40, 33, 1.0)])
+def test_cq_small_values(ctx, oracle_lib, rng, interp, ny, nx, cut):
+    o = oracle_lib
+    _, km, mq = small_detector(ny, nx, 6e-4)
+    npix = ny * nx
+    s = o.small_cq_mesh_shape(mq, 41)
+    s.max_q = np.float32(cut) * s.max_q
+    for name, I, k, mult in _cases(rng, npix, km):
+        want = np.zeros(s.size_ab * s.size_ab * s.size_c, np.uint64)
+        o.lib().iaco_cq_small(o.p(I), o.p(k), npix, s, interp, mult, 0, npix, o.p(want))
+        for fast in (0, nx):
+            out = _dev(np.zeros(want.size, np.int64))
+            ctx.cq_small(_dev(I), _dev(k), npix, to_capi_shape(s), interp, mult, out, fast_size=fast)
+            np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=f"{name} {fast}")
