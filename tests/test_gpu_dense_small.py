@@ -1,4 +1,4 @@
-"""Dense C(q) tiles whose values stay below 2^23 (their own kernels'
+"""Dense C(q) and AC1D tiles whose values stay below 2^23 (their own kernels'
 path) next to tiles that leave it, bit for bit against the oracle: values at
 the limit, negative intensities, masked pixels whose k is far outside the mesh,
 MaxQ cuts, ragged tiles, Multiplicators that are no integers or no floats."""
@@ -53,3 +53,24 @@ def test_cq_small_values(ctx, oracle_lib, rng, interp, ny, nx, cut):
             out = _dev(np.zeros(want.size, np.int64))
             ctx.cq_small(_dev(I), _dev(k), npix, to_capi_shape(s), interp, mult, out, fast_size=fast)
             np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=f"{name} {fast}")
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+@pytest.mark.parametrize("ny,nx,size,cut", [(16, 16, 3, 1.0), (17, 31, 300, 0.6), (40, 33, 1000, 1.0)])
+def test_ac1d_small_values(ctx, oracle_lib, rng, interp, ny, nx, size, cut):
+    from incohautocorrelate_b200 import capi
+    o = oracle_lib
+    _, km, mq = small_detector(ny, nx, 6e-4)
+    npix = ny * nx
+    so, sh = o.ac1d_shape(mq, size), capi.ac1d_shape(mq, size)
+    max_q = np.float32(cut * sh.max_q)
+    for wrap in (1.0, 0.7):  # 0.7: bins past the histogram wrap around it
+        for s in (so, sh):
+            s.max_q = max_q
+            s.dq_per_step = np.float32(max_q / (size - 1.5) * wrap)
+        for name, I, k, mult in _cases(rng, npix, km):
+            want = np.zeros(sh.size, np.uint64)
+            o.lib().iaco_ac1d_cq(o.p(I), o.p(k), npix, so, interp, mult, 0, npix, o.p(want))
+            out = _dev(np.zeros(want.size, np.int64))
+            ctx.ac1d_cq(_dev(I), _dev(k), npix, sh, interp, mult, out)
+            np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=f"{name} {wrap}")
