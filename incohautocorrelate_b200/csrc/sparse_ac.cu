@@ -255,39 +255,62 @@ __global__ void __cluster_dims__(PLAN_CTAS, 1, 1) __launch_bounds__(PLAN_THREADS
 }
 
 // a small batch planned by the CTA itself in shared memory (every thread of
-// the block): s_off gets nframes + 1 starts; returns the header
+// the block): s_off gets nframes + 1 starts; returns the header.  The sums and the
+// scan take the whole block: by one warp, with 64-bit shared adds, 200 frames took
+// 9 us longer.
 __device__ __forceinline__ PlanHeader plan_direct(const WalkArgs &a, uint32_t warps, unsigned long long *s_off,
-                                                  unsigned long long *s_pairs)
+                                                  unsigned long long *warp_sums)
 {
-    const uint32_t tid = threadIdx.x;
-    if (tid == 0) *s_pairs = 0ull;
-    __syncthreads();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    PlanHeader h;
+    h.next = 0u;
+    if (a.nframes <= 32) {  // each warp by itself, one barrier
+        const uint32_t n = lane < a.nframes ? (uint32_t)(a.offsets[lane + 1] - a.offsets[lane]) : 0u;
+        h.pairs = frame_pairs(n);
+        for (int o = 16; o; o >>= 1) h.pairs += __shfl_xor_sync(0xffffffffu, h.pairs, o);
+        h.steps = batch_steps(h.pairs, warps, a.steps_max);
+        unsigned long long incl = lane < a.nframes ? frame_cost(n, h.steps) : 0ull;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long u = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += u;
+        }
+        if (w == 0 && lane < a.nframes) s_off[lane + 1] = incl;
+        if (tid == 0) s_off[0] = 0ull;
+        __syncthreads();
+        h.cost = __shfl_sync(0xffffffffu, incl, 31);
+        return h;
+    }
+    unsigned long long pairs = 0;
     for (uint32_t f = tid; f < a.nframes; f += blockDim.x) {
         const uint32_t n = (uint32_t)(a.offsets[f + 1] - a.offsets[f]);
         s_off[f + 1] = n;
-        if (n > 1) atomicAdd(s_pairs, frame_pairs(n));
+        pairs += frame_pairs(n);
     }
-    __syncthreads();
-    PlanHeader h;
-    h.pairs = *s_pairs;
+    h.pairs = block_sum_u64(pairs, warp_sums);
     h.steps = batch_steps(h.pairs, warps, a.steps_max);
-    h.next = 0u;
-    if (tid < 32) {
-        unsigned long long run = 0;
-        for (uint32_t c0 = 0; c0 < a.nframes; c0 += 32) {
-            const uint32_t f = c0 + tid;
-            unsigned long long incl = f < a.nframes ? frame_cost((uint32_t)s_off[f + 1], h.steps) : 0ull;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long u = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)tid >= o) incl += u;
-            }
-            if (f < a.nframes) s_off[f + 1] = run + incl;
-            run += __shfl_sync(0xffffffffu, incl, 31);
+    unsigned long long run = 0;
+    for (uint32_t c0 = 0; c0 < a.nframes; c0 += blockDim.x) {
+        const uint32_t f = c0 + tid;
+        unsigned long long incl = f < a.nframes ? frame_cost((uint32_t)s_off[f + 1], h.steps) : 0ull;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long u = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += u;
         }
-        if (tid == 0) s_off[0] = 0ull;
+        __syncthreads();
+        if (lane == 31) warp_sums[w] = incl;
+        __syncthreads();
+        unsigned long long before = 0, all = 0;
+        for (uint32_t k = 0; k < blockDim.x / 32; k++) {
+            const unsigned long long s = warp_sums[k];
+            before += k < w ? s : 0ull;
+            all += s;
+        }
+        if (f < a.nframes) s_off[f + 1] = run + before + incl;
+        run += all;
     }
+    if (tid == 0) s_off[0] = 0ull;
     __syncthreads();
-    h.cost = s_off[a.nframes];
+    h.cost = run;
     return h;
 }
 
@@ -821,7 +844,7 @@ __global__ void __launch_bounds__(pair_threads(DMAP, I1, I2), 1) sparse_pairs_ke
 {
     constexpr bool FAST = DMAP == 0 || I1 == 0;
     __shared__ unsigned long long s_off[PAIR_DIRECT + 1];
-    __shared__ unsigned long long s_pairs;
+    __shared__ unsigned long long s_sums[32];
     __shared__ uint32_t s_next, s_taken, s_worst[32];
     __shared__ uint32_t s_flags[PAIR_DIRECT];
     extern __shared__ uint32_t s_box[];  // (box_r + 1) x box_w x box_w low words, [ss][ms][fs]
@@ -830,7 +853,7 @@ __global__ void __launch_bounds__(pair_threads(DMAP, I1, I2), 1) sparse_pairs_ke
     const uint32_t nthr = blockDim.x;
     const int lane = threadIdx.x & 31;
     const unsigned long long *off = a.walk.head ? a.walk.cost_off : s_off;
-    const PlanHeader h = a.walk.head ? *a.walk.head : plan_direct(a.walk, gridDim.x * (nthr / 32), s_off, &s_pairs);
+    const PlanHeader h = a.walk.head ? *a.walk.head : plan_direct(a.walk, gridDim.x * (nthr / 32), s_off, s_sums);
     const Share share = cta_share(h, a.walk.head != nullptr);
     if (share.x0 >= share.x1) return;  // a CTA without work (uniform over the block)
     if (threadIdx.x == 0) s_next = s_taken = 0u;
@@ -943,60 +966,6 @@ __global__ void __launch_bounds__(pair_threads(DMAP, I1, I2), 1) sparse_pairs_ke
 }
 
 // ---------------------------------------------------------------------------
-// planner: tiles per frame, exclusive scan, queue reset (one CTA)
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ unsigned long long frame_tiles(const uint64_t *off, uint32_t f,
-                                                          uint32_t tile_pairs)
-{
-    const unsigned long long n = off[f + 1] - off[f];
-    if (n == 0) return 0;
-    const unsigned long long pairs = n * (n - 1) / 2;
-    const unsigned long long t = (pairs + tile_pairs - 1) / tile_pairs;
-    return t > 0 ? t : 1;
-}
-
-__global__ void __launch_bounds__(PLAN_THREADS)
-    ac1d_plan_kernel(const uint64_t *__restrict__ off, uint32_t nframes, uint32_t tile_pairs,
-                       unsigned long long *__restrict__ tile_off, unsigned long long *queue)
-{
-    __shared__ unsigned long long warp_sums[PLAN_THREADS / 32];
-    const uint32_t tid = threadIdx.x;
-    const uint32_t chunk = (nframes + PLAN_THREADS - 1) / PLAN_THREADS;
-    const uint32_t f0 = min(nframes, tid * chunk), f1 = min(nframes, f0 + chunk);
-    unsigned long long local = 0;
-    for (uint32_t f = f0; f < f1; f++) local += frame_tiles(off, f, tile_pairs);
-    // block-wide exclusive scan of the per-thread sums
-    const int lane = tid & 31, w = tid >> 5;
-    unsigned long long incl = local;
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_sums[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-        unsigned long long v = warp_sums[lane];
-        unsigned long long s = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long u = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += u;
-        }
-        warp_sums[lane] = s - v;  // exclusive warp prefix
-    }
-    __syncthreads();
-    unsigned long long run = warp_sums[w] + incl - local;
-    for (uint32_t f = f0; f < f1; f++) {
-        tile_off[f] = run;
-        run += frame_tiles(off, f, tile_pairs);
-    }
-    if (tid == PLAN_THREADS - 1) {
-        tile_off[nframes] = warp_sums[w] + incl;
-        *queue = 0ull;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // fold: full[fs, ms, ss + C] += half; full[2C - fs, 2C - ms, C - ss] += half
 // for ss > 0 (IAC/Detector.cpp:1147-1170).  Every full-mesh voxel receives
 // exactly one half-mesh voxel, so plain read-modify-write suffices.
@@ -1039,12 +1008,23 @@ __global__ void sparse_fold_kernel(const unsigned long long *__restrict__ half, 
 // double histogram of Size bins; the factor 2 also doubles the self pair.
 // These floats are whole numbers for photon counts (nearest): those are summed
 // in uint64, exactly, so the double totals equal the reference's sequential
-// double sums bit for bit.  Any other value is summed with double atomics,
-// whose order differs from the reference's loop by rounding only.
+// double sums bit for bit.  Fractions from counts (linear) are multiples of
+// fix_top 2^-23 past the first bins, because |q| / dq has 24 bits and some of them
+// go to the bin; those are summed in these units, exactly too: 32-bit shared adds
+// are native, while a double add in shared memory is a loop of compare-and-swaps.
+// Adding and taking off fix_top tells whether a value is one.  The rest is summed
+// with double atomics, whose order differs from the reference's loop by rounding
+// only, as are all fractions when the histograms leave no room for the
+// fixed-point one.
 //
-// The histograms live in shared memory for the whole launch; the work queue
-// and the pair enumeration are the pair kernel's.  A tile belongs to one
-// frame, so the route branch is uniform across the CTA.
+// The histograms live in shared memory for the whole launch.  The walk over the
+// batch and its planner are the pair kernel's: a warp's lanes take consecutive
+// photons i and step through partners two at a time, the squared distances in
+// f32x2, |q| / dq by the two-word reciprocal; the order of a pair's photons
+// changes neither |q| nor the value.  A unit belongs to one frame, so the route
+// branch is uniform across the warp.  Issue-bound (80 %, 110 instructions a pair):
+// 20 000 frames (2.2e8 pairs, 2048 bins) 1578 -> 857 us linear, 979 -> 590 nearest;
+// in double adds the linear walk took 1100.
 // ---------------------------------------------------------------------------
 // b % n without the division when b < n (bins past the histogram are rare)
 __device__ __forceinline__ uint32_t wrap_bin(uint32_t b, uint32_t n)
@@ -1054,17 +1034,18 @@ __device__ __forceinline__ uint32_t wrap_bin(uint32_t b, uint32_t n)
 }
 
 struct AC1DArgs {
-    const float4 *__restrict__ photons;
-    const uint64_t *__restrict__ offsets;
-    const unsigned long long *__restrict__ tile_off;  // nframes + 1
-    unsigned long long *queue;
+    WalkArgs walk;
     DeviceCounters *counters;
-    uint32_t nframes;
-    uint32_t tile_pairs;
     double mult;
     float maxq, dqdx;
+    Divisor by_dq;
+    float neg_zero;
     uint32_t vecsize;   // device-route bins (VecSize)
     uint32_t size;      // host-route bins (Shape.Size; 0 when no frame takes the host route)
+    int divide;         // dq is too large or small for by_dq
+    int fixed;          // the fixed-point histogram has room
+    float fix_top;      // its values are below this, in units of fix_top 2^-23
+    uint32_t fix_mask;  // the units' fraction bits
     float det_pixels;   // (float) detector pixel count, for the route choice
     int route;          // -1: the reference's choice per frame, 0: host route, 1: device route
     unsigned long long *dev_out;  // vecsize words
@@ -1073,157 +1054,240 @@ struct AC1DArgs {
 };
 
 // shared-memory histograms of one CTA: 64-bit counters as split 32-bit words
-// (shared_add_u64_split), host-route fractions as doubles
+// (shared_add_u64_split), host-route fractions in units of 2^-32 or as doubles
 struct AC1DHist {
     uint32_t *dev_lo, *dev_hi;  // vecsize words each
-    uint32_t *int_lo, *int_hi;  // size words each
-    double *frac;               // size doubles
+    unsigned long long *whole;  // size split words, then size doubles
+    uint32_t *fix_lo, *fix_hi;  // size words each (if fixed)
 };
 
-// host-route value v (>= 0) into bin b
-__device__ __forceinline__ void host_route_add(const AC1DArgs &b, const AC1DHist &h,
+__device__ __forceinline__ uint32_t shared_add32(uint32_t at, uint32_t v)
+{
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
+    return old;
+}
+// host-route value v (>= 0) into a bin of the whole-number histogram (split words)
+// and the doubles behind it
+__device__ __forceinline__ void host_route_add(unsigned long long *whole, uint32_t size, DeviceCounters *counters,
                                                uint32_t bin, float v)
 {
-    if (bin >= b.size) {  // only for inconsistent MaxQ / dq; the reference writes out of bounds
-        atomicAdd(&b.counters->out_of_mesh, 1ull);
+    if (bin >= size) {  // only for inconsistent MaxQ / dq; the reference writes out of bounds
+        atomicAdd(&counters->out_of_mesh, 1ull);
         return;
     }
     if (v == 0.0f) return;
+    uint32_t *lo = reinterpret_cast<uint32_t *>(whole), *hi = lo + size;
+    double *frac = reinterpret_cast<double *>(whole + size);
     if (v > 0.0f && v < 8388608.0f) {  // the usual case, without conversion-unit instructions
         const float t = __fadd_rz(v, 8388608.0f);  // 2^23 + floor(v)
         if (fsub(t, 8388608.0f) == v)
-            shared_add_u64_split(h.int_lo, h.int_hi, bin, (unsigned long long)(uint32_t)(__float_as_int(t) - TWO23_BITS));
+            shared_add_u64_split(lo, hi, bin, (unsigned long long)(uint32_t)(__float_as_int(t) - TWO23_BITS));
         else
-            atomicAdd(&h.frac[bin], (double)v);
+            atomicAdd(&frac[bin], (double)v);
         return;
     }
     if (v == truncf(v) && v < 1.8e19f)
-        shared_add_u64_split(h.int_lo, h.int_hi, bin, (unsigned long long)__float2ull_rz(v));
+        shared_add_u64_split(lo, hi, bin, (unsigned long long)__float2ull_rz(v));
     else
-        atomicAdd(&h.frac[bin], (double)v);
+        atomicAdd(&frac[bin], (double)v);
+}
+// twice floor(x) of a device-route value into bin
+__device__ __forceinline__ void device_route_add(const AC1DArgs &b, const AC1DHist &h, uint32_t bin, double x)
+{
+    unsigned long long w;
+    if ((uint32_t)__double2hiint(x) < 0x41E00000u)  // [0, 2^31): without the 64-bit conversion
+        w = (uint32_t)__double2loint(__dadd_rz(x, 4503599627370496.0));
+    else
+        w = d2u64(x);
+    if (w) shared_add_u64_split(h.dev_lo, h.dev_hi, wrap_bin(bin, b.vecsize), 2ull * w);
 }
 
+// 20 000 frames, linear, by threads x CTAs per SM: 512 x 2 857 us, 512 x 3 823, 768 x 2
+// 817, 1024 x 1 855; 200 frames 39, 57, 47 and 52: a short batch pays for each CTA.
+constexpr int AC1D_THREADS = 512, AC1D_PER_SM = 2;
+// batches planned by the CTAs themselves: 1000 frames 79 us, with the planner's launch 87
+constexpr uint32_t AC1D_DIRECT = 1024;
 template <int INTERP>
-__global__ void __launch_bounds__(256) ac1d_sparse_kernel(const AC1DArgs a)
+__global__ void __launch_bounds__(AC1D_THREADS, AC1D_PER_SM) ac1d_sparse_kernel(const AC1DArgs a)
 {
+    __shared__ unsigned long long s_off[AC1D_DIRECT + 1];
+    __shared__ unsigned long long s_sums[32];
+    __shared__ uint32_t s_next, s_taken;
     extern __shared__ unsigned long long hist[];
-    const AC1DArgs &b = a;
     AC1DHist h;
     h.dev_lo = reinterpret_cast<uint32_t *>(hist);
-    h.dev_hi = h.dev_lo + b.vecsize;
-    h.int_lo = h.dev_hi + b.vecsize;
-    h.int_hi = h.int_lo + b.size;
-    h.frac = reinterpret_cast<double *>(hist + b.vecsize + b.size);
-    __shared__ unsigned long long s_tile;
-    __shared__ uint32_t s_frame;
-    const uint32_t words = b.vecsize + 2 * b.size;
-    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) hist[i] = 0;  // 0 bits = +0.0
-    const unsigned long long ntiles = a.tile_off[a.nframes];
+    h.dev_hi = h.dev_lo + a.vecsize;
+    h.whole = hist + a.vecsize;
+    h.fix_lo = reinterpret_cast<uint32_t *>(hist + a.vecsize + 2 * a.size);
+    h.fix_hi = h.fix_lo + a.size;
     const uint32_t nthr = blockDim.x;
-    const float maxq = b.maxq, dqdx = b.dqdx;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned long long t = atomicAdd(a.queue, 1ull);
-            s_tile = t;
-            if (t < ntiles) {
-                uint32_t lo = 0, hi = a.nframes;
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (a.tile_off[mid] <= t) lo = mid; else hi = mid;
-                }
-                s_frame = lo;
-            }
-        }
-        __syncthreads();
-        const unsigned long long t = s_tile;
-        if (t >= ntiles) break;
-        const uint32_t f = s_frame;
-        const uint64_t base = a.offsets[f];
-        const uint32_t n = (uint32_t)(a.offsets[f + 1] - base);
-        const unsigned long long chunk = t - a.tile_off[f];
-        const float4 *__restrict__ P = a.photons + base;
-        // SHLsizeQuot < 0.0075f (IAC/AC1D.cpp:251-253), in the reference's float arithmetic
-        const bool host =
-            b.route == 0 || (b.route < 0 && __fdiv_rn(__uint2float_rn(n), b.det_pixels) < 0.0075f);
-        if (chunk == 0)  // self pairs: q = 0, bin 0 (linear: bin 0 gets all of it, bin 1 nothing)
-            for (uint32_t i = threadIdx.x; i < n; i += nthr) {
-                const float w = P[i].w;
+    const unsigned long long *off = a.walk.head ? a.walk.cost_off : s_off;
+    const PlanHeader head = a.walk.head ? *a.walk.head : plan_direct(a.walk, gridDim.x * (nthr / 32), s_off, s_sums);
+    const Share share = cta_share(head, a.walk.head != nullptr);
+    if (share.x0 >= share.x1) return;  // a CTA without work (uniform over the block)
+    if (threadIdx.x == 0) s_next = s_taken = 0u;
+    const uint32_t words = a.vecsize + (a.fixed ? 3 : 2) * a.size;
+    for (uint32_t i = threadIdx.x; i < words; i += nthr) hist[i] = 0;  // 0 bits = +0.0
+    __syncthreads();
+    const uint32_t whole = (uint32_t)__cvta_generic_to_shared(h.whole), 
+                   // without room every pair adds 0, at a word that exists
+                   fixed = a.fixed ? (uint32_t)__cvta_generic_to_shared(h.fix_lo) : whole;
+    const uint32_t fix_bins = a.fixed ? a.size - 1 : 0u;  // a pair's first bin below this: both exist
+    const float2 nz = make_float2(a.neg_zero, a.neg_zero);
+    const float4 *__restrict__ P = nullptr;
+    uint32_t n = 0;
+    bool host = false;
+    unsigned long long self_int = 0, self_dev = 0;  // this lane's self pairs: q = 0, bin 0
+    walk_share(
+        a.walk, head, off, share, a.walk.head ? &a.walk.head->next : &s_next, &s_taken,
+        [&](uint32_t, uint64_t base, uint32_t nf) {
+            P = a.walk.photons + base;
+            n = nf;
+            // SHLsizeQuot < 0.0075f (IAC/AC1D.cpp:251-253), in the reference's float arithmetic
+            host = a.route == 0 || (a.route < 0 && __fdiv_rn(__uint2float_rn(n), a.det_pixels) < 0.0075f);
+        },
+        [&](uint32_t i, uint32_t c, bool active, uint32_t, uint32_t L) {
+            uint32_t d0;
+            int steps;
+            chunk_steps(n, i, c, L, active, d0, steps);
+            const float4 A = P[i];
+            if (active && c == 0) {  // linear: bin 0 gets all of it, bin 1 nothing
                 if (host) {
-                    host_route_add(b, h, 0, fmul(2.0f, fmul(w, w)));
+                    const float v = fmul(2.0f, fmul(A.w, A.w));
+                    if (v == truncf(v) && v < 1.8e19f)
+                        self_int += __float2ull_rz(v);
+                    else
+                        host_route_add(h.whole, a.size, a.counters, 0, v);
                 } else {
-                    const double v = (double)w;
-                    const unsigned long long u = d2u64(dmul(dmul(v, v), a.mult));
-                    if (u) shared_add_u64_split(h.dev_lo, h.dev_hi, 0, u);
+                    const double v = (double)A.w;
+                    self_dev += d2u64(dmul(dmul(v, v), a.mult));
                 }
             }
-        const unsigned long long npairs = (unsigned long long)n * (n - 1) / 2;
-        const unsigned long long p0 = chunk * a.tile_pairs;
-        const unsigned long long p1 = min(npairs, p0 + a.tile_pairs);
-        if (p0 + threadIdx.x < p1) {
-            unsigned long long l = p0 + threadIdx.x;
-            uint32_t d = (uint32_t)(l / n) + 1;
-            uint32_t i = (uint32_t)(l - (unsigned long long)(d - 1) * n);
-            const uint32_t dq = nthr / n, dr = nthr % n;
-            for (; l < p1; l += nthr) {
-                uint32_t j = i + d;
-                if (j >= n) j -= n;
-                const float4 A = P[min(i, j)], B = P[max(i, j)];
-                const float dx = fsub(A.x, B.x), dy = fsub(A.y, B.y), dz = fsub(A.z, B.z);
-                float q = __fsqrt_rn(fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fmul(dz, dz)));
-                if (!(q > maxq)) {
-                    q = __fdiv_rn(q, dqdx);
-                    if (host) {
-                        const float pv = fmul(A.w, B.w);
-                        if (INTERP == 0) {
-                            // (uint)floor(q + 0.5) in double, as floor(fl(q + 0.49999997f)) for q < 2^23
-                            uint32_t iq;
-                            floor_small(fadd(q, 0.49999997f), iq);
-                            host_route_add(b, h, iq, fmul(2.0f, pv));
-                        } else {
-                            uint32_t iq;  // q = |q| / dq <= MaxQ / dq < 2^23
-                            const float fq = floor_small(q, iq);
-                            const float sep = fsub(q, fq);
-                            host_route_add(b, h, iq, fmul(2.0f, fmul(pv, fsub(1.0f, sep))));
-                            host_route_add(b, h, iq + 1, fmul(2.0f, fmul(pv, sep)));
+            uint32_t j = i + d0;
+            if (j >= n) j -= n;
+            for (int k = 0; k < (int)L; k += 2) {
+                const float4 B0 = P[j];
+                if (++j == n) j = 0;
+                const float4 B1 = P[j];
+                if (++j == n) j = 0;
+                const float2 dx = f2sub(make_float2(A.x, A.x), make_float2(B0.x, B1.x)),
+                             dy = f2sub(make_float2(A.y, A.y), make_float2(B0.y, B1.y)),
+                             dz = f2sub(make_float2(A.z, A.z), make_float2(B0.z, B1.z));
+                const float2 s = f2add(f2add(f2fma(dx, dx, nz), f2fma(dy, dy, nz)), f2fma(dz, dz, nz));
+                const float2 r = make_float2(__fsqrt_rn(s.x), __fsqrt_rn(s.y));
+                float2 qq;
+                if (a.divide)
+                    qq = make_float2(__fdiv_rn(r.x, a.dqdx), __fdiv_rn(r.y, a.dqdx));
+                else
+                    qq = f2div(r, a.by_dq);
+                const bool on[2] = {k < steps && !(r.x > a.maxq), k + 1 < steps && !(r.y > a.maxq)};
+                const float q[2] = {qq.x, qq.y}, bw[2] = {B0.w, B1.w};
+                if (INTERP == 0 && host) {
+                    uint32_t bin[2], u[2], old[2];
+                    float v[2];
+                    bool rare[2];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        // (uint)floor(q + 0.5) in double, as floor(fl(q + 0.49999997f)) for q < 2^23
+                        floor_small(fadd(q[e], 0.49999997f), bin[e]);
+                        v[e] = fmul(2.0f, fmul(A.w, bw[e]));
+                        const bool fast = floor_small(v[e], u[e]) == v[e] && u[e] < (1u << 23) && bin[e] < a.size;
+                        rare[e] = on[e] && !fast;
+                        u[e] = on[e] && fast ? u[e] : 0u;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; e++) old[e] = shared_add32(whole + (u[e] ? 4u * bin[e] : 0u), u[e]);
+                    if (old[0] + u[0] < old[0]) shared_add32(whole + 4u * (a.size + bin[0]), 1u);
+                    if (old[1] + u[1] < old[1]) shared_add32(whole + 4u * (a.size + bin[1]), 1u);
+                    if (rare[0] || rare[1]) {
+#pragma unroll 1
+                        for (int e = 0; e < 2; e++)
+                            if (e ? rare[1] : rare[0])
+                                host_route_add(h.whole, a.size, a.counters, e ? bin[1] : bin[0], e ? v[1] : v[0]);
+                    }
+                } else if (INTERP == 0) {
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        uint32_t iq;
+                        floor_small(fadd(q[e], 0.49999997f), iq);  // as above
+                        if (on[e]) device_route_add(a, h, iq, dmul(dmul((double)A.w, (double)bw[e]), a.mult));
+                    }
+                } else if (host) {
+                    uint32_t at[2], bin[2], u[4];
+                    float v[4];
+                    bool rare[2], c[4];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        // q = |q| / dq <= MaxQ / dq < 2^23
+                        const float fq = floor_small(q[e], bin[e]);
+                        const float sep = fsub(q[e], fq), pv = fmul(A.w, bw[e]);
+                        v[2 * e] = fmul(2.0f, fmul(pv, fsub(1.0f, sep)));
+                        v[2 * e + 1] = fmul(2.0f, fmul(pv, sep));
+                        const bool in = on[e] && bin[e] < fix_bins;
+                        at[e] = in ? fixed + 4u * bin[e] : fixed;  // off: adds 0
+                        bool ok[2];
+#pragma unroll
+                        for (int m = 0; m < 2; m++) {
+                            const float x = v[2 * e + m], s = fadd(x, a.fix_top);
+                            const uint32_t w = __float_as_uint(s) - __float_as_uint(a.fix_top);
+                            // below the top, exact, and no whole number
+                            ok[m] = in && w < (1u << 23) && fsub(s, a.fix_top) == x && (w & a.fix_mask) != 0;
+                            u[2 * e + m] = ok[m] ? w : 0u;
                         }
-                    } else {
-                        const double val = dmul((double)A.w, (double)B.w);
-                        if (INTERP == 0) {
-                            uint32_t iq;  // (uint)floor(q + 0.5), as above
-                            floor_small(fadd(q, 0.49999997f), iq);
-                            const uint32_t sc = wrap_bin(iq, b.vecsize);
-                            const unsigned long long w = d2u64(dmul(val, a.mult));
-                            if (w) shared_add_u64_split(h.dev_lo, h.dev_hi, sc, 2ull * w);
-                        } else {
-                            uint32_t iq;
-                            const float fq = floor_small(q, iq);
-                            const double sep = (double)fsub(q, fq);
-                            const unsigned long long w1 = d2u64(dmul(dmul(val, dsub(1.0, sep)), a.mult));
-                            const unsigned long long w2 = d2u64(dmul(dmul(val, sep), a.mult));
-                            if (w1) shared_add_u64_split(h.dev_lo, h.dev_hi, wrap_bin(iq, b.vecsize), 2ull * w1);
-                            if (w2) shared_add_u64_split(h.dev_lo, h.dev_hi, wrap_bin(iq + 1, b.vecsize), 2ull * w2);
+                        rare[e] = on[e] && !(ok[0] && ok[1]);
+                    }
+#pragma unroll
+                    for (int m = 0; m < 4; m++) c[m] = shared_add32(at[m >> 1] + 4u * (m & 1), u[m]) + u[m] < u[m];
+                    if (c[0] | c[1] | c[2] | c[3]) {
+#pragma unroll
+                        for (int m = 0; m < 4; m++)
+                            if (c[m]) shared_add32(at[m >> 1] + 4u * (m & 1) + 4u * a.size, 1u);
+                    }
+                    if (rare[0] || rare[1]) {
+#pragma unroll 1
+                        for (int m = 0; m < 4; m++) {
+                            const bool second = m >= 2;
+                            const uint32_t w = second ? (m & 1 ? u[3] : u[2]) : (m & 1 ? u[1] : u[0]);
+                            if (w == 0 && (second ? on[1] : on[0]))
+                                host_route_add(h.whole, a.size, a.counters, (second ? bin[1] : bin[0]) + (m & 1),
+                                               second ? (m & 1 ? v[3] : v[2]) : (m & 1 ? v[1] : v[0]));
                         }
                     }
-                }
-                i += dr;
-                d += dq;
-                if (i >= n) {
-                    i -= n;
-                    d += 1;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        uint32_t iq;
+                        const float fq = floor_small(q[e], iq);
+                        if (!on[e]) continue;
+                        const double sep = (double)fsub(q[e], fq), val = dmul((double)A.w, (double)bw[e]);
+                        device_route_add(a, h, iq, dmul(dmul(val, dsub(1.0, sep)), a.mult));
+                        device_route_add(a, h, iq + 1, dmul(dmul(val, sep), a.mult));
+                    }
                 }
             }
-        }
-        __syncthreads();
+        });
+    uint32_t *int_lo = reinterpret_cast<uint32_t *>(h.whole), *int_hi = int_lo + a.size;
+    const double *frac = reinterpret_cast<double *>(h.whole + a.size);
+    for (int o = 16; o; o >>= 1) {
+        self_int += __shfl_xor_sync(0xffffffffu, self_int, o);
+        self_dev += __shfl_xor_sync(0xffffffffu, self_dev, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (self_int) shared_add_u64_split(int_lo, int_hi, 0, self_int);
+        if (self_dev) shared_add_u64_split(h.dev_lo, h.dev_hi, 0, self_dev);
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < b.vecsize; i += blockDim.x) {
+    for (uint32_t i = threadIdx.x; i < a.vecsize; i += nthr) {
         const unsigned long long v = split_word(h.dev_lo, h.dev_hi, i);
-        if (v) atomicAdd(&b.dev_out[i], v);
+        if (v) atomicAdd(&a.dev_out[i], v);
     }
-    for (uint32_t i = threadIdx.x; i < b.size; i += blockDim.x) {
-        const unsigned long long v = split_word(h.int_lo, h.int_hi, i);
-        if (v) atomicAdd(&b.int_out[i], v);
-        if (h.frac[i] != 0.0) atomicAdd(&b.frac_out[i], h.frac[i]);
+    for (uint32_t i = threadIdx.x; i < a.size; i += nthr) {
+        const unsigned long long v = split_word(int_lo, int_hi, i);
+        if (v) atomicAdd(&a.int_out[i], v);
+        double f = frac[i];
+        if (a.fixed) f = dadd(f, dmul(__ull2double_rn(split_word(h.fix_lo, h.fix_hi, i)), (double)a.fix_top * 0x1p-23));
+        if (f != 0.0) atomicAdd(&a.frac_out[i], f);
     }
 }
 
@@ -1409,27 +1473,45 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
     const size_t table_bytes = ((sizeof(unsigned long long) * ((size_t)nframes + 1) + 127) / 128) * 128;
     iac_status st = stream_scratch(ctx, stream, SLOT_TILES, table_bytes + 128 + nframes, &scratch);
     if (st != IAC_OK) return st;
-    unsigned long long *tile_off = (unsigned long long *)scratch;
-    unsigned long long *queue = (unsigned long long *)((char *)scratch + table_bytes);
     cudaStream_t s = as_stream(stream);
-    ac1d_plan_kernel<<<1, PLAN_THREADS, 0, s>>>(d_off, nframes, tun.tile_pairs, tile_off, queue);
-    IAC_LAUNCHED(ctx);
-    IAC_CUDA(cudaGetLastError());
     AC1DArgs a = b;
-    a.photons = reinterpret_cast<const float4 *>(d_photons);
-    a.offsets = d_off;
-    a.tile_off = tile_off;
-    a.queue = queue;
+    // the fixed-point histogram where two CTAs an SM (one, for large shapes) still fit
+    const size_t plain = sizeof(unsigned long long) * ((size_t)b.vecsize + 2 * (size_t)b.size),
+                 more = sizeof(unsigned long long) * b.size;
+    a.fixed = interp == 1 && b.size > 1 && plain + more <= (216u << 10);
+    const size_t smem = plain + (a.fixed ? more : 0);
+    // |q| / dq from 2^e on is a multiple of 2^(e - 23): with 2^(e + 1) for the top, the
+    // counts' values are too; the first 2^e bins, 1/32 of them, see few of the pairs
+    int e = 2;
+    while (e < 6 && (64u << (e - 1)) <= b.size) e++;
+    a.fix_top = (float)(2u << e);
+    a.fix_mask = (1u << (22 - e)) - 1;
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(AC1D_PER_SM, (208u << 10) / std::max<size_t>(smem, 1)));
+    const int grid = ctx->sm_count * per_sm;
+    const bool direct = nframes <= AC1D_DIRECT;
+    unsigned long long *cost_off = (unsigned long long *)scratch;
+    PlanHeader *head = (PlanHeader *)((char *)scratch + table_bytes);
+    a.walk.photons = reinterpret_cast<const float4 *>(d_photons);
+    a.walk.offsets = d_off;
+    a.walk.head = direct ? nullptr : head;
+    a.walk.cost_off = cost_off;
+    a.walk.nframes = nframes;
+    a.walk.steps_max = std::min(PAIR_STEPS_MAX, std::max(1u, tun.tile_pairs / 32));
     a.counters = ctx->d_counters;
-    a.nframes = nframes;
-    a.tile_pairs = tun.tile_pairs;
+    a.by_dq = make_divisor(b.dqdx);
+    a.divide = !(b.dqdx > 1e-30f && b.dqdx < 1e30f);
+    a.neg_zero = -0.0f;
     a.mult = mult;
-    const size_t smem = sizeof(unsigned long long) * ((size_t)b.vecsize + 2 * (size_t)b.size);
+    if (!direct) {  // without the count check
+        sparse_plan_kernel<<<PLAN_CTAS, PLAN_THREADS, 0, s>>>(d_off, nframes, a.walk.steps_max,
+                                                              (uint32_t)(grid * AC1D_THREADS / 32), cost_off, head,
+                                                              a.walk.photons, nullptr, 0.0f, nullptr);
+        IAC_LAUNCHED(ctx);
+        IAC_CUDA(cudaGetLastError());
+    }
     auto k = interp == 0 ? ac1d_sparse_kernel<0> : ac1d_sparse_kernel<1>;
     IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // as many persistent CTAs as fit: four per SM, fewer when the histograms are large
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (200u << 10) / std::max<size_t>(smem, 1)));
-    k<<<ctx->sm_count * per_sm, 256, smem, s>>>(a);
+    k<<<grid, AC1D_THREADS, smem, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
     return IAC_OK;
