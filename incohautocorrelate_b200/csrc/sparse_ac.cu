@@ -1023,8 +1023,9 @@ __global__ void sparse_fold_kernel(const unsigned long long *__restrict__ half, 
 // f32x2, |q| / dq by the two-word reciprocal; the order of a pair's photons
 // changes neither |q| nor the value.  A unit belongs to one frame, so the route
 // branch is uniform across the warp.  Issue-bound (80 %, 110 instructions a pair):
-// 20 000 frames (2.2e8 pairs, 2048 bins) 1578 -> 857 us linear, 979 -> 590 nearest;
-// in double adds the linear walk took 1100.
+// 20 000 frames (2.2e8 pairs, 2048 bins) 1578 -> 910 us linear, 979 -> 590 nearest;
+// with double adds the linear walk took 1100.  Device route, 2 000 frames of 230
+// photons, 950 bins: 455 -> 288 us linear, 347 -> 239 nearest.
 // ---------------------------------------------------------------------------
 // b % n without the division when b < n (bins past the histogram are rare)
 __device__ __forceinline__ uint32_t wrap_bin(uint32_t b, uint32_t n)
@@ -1095,11 +1096,7 @@ __device__ __forceinline__ void host_route_add(unsigned long long *whole, uint32
 // twice floor(x) of a device-route value into bin
 __device__ __forceinline__ void device_route_add(const AC1DArgs &b, const AC1DHist &h, uint32_t bin, double x)
 {
-    unsigned long long w;
-    if ((uint32_t)__double2hiint(x) < 0x41E00000u)  // [0, 2^31): without the 64-bit conversion
-        w = (uint32_t)__double2loint(__dadd_rz(x, 4503599627370496.0));
-    else
-        w = d2u64(x);
+    const unsigned long long w = d2u64(x);
     if (w) shared_add_u64_split(h.dev_lo, h.dev_hi, wrap_bin(bin, b.vecsize), 2ull * w);
 }
 
@@ -1109,7 +1106,7 @@ constexpr int AC1D_THREADS = 512, AC1D_PER_SM = 2;
 // batches planned by the CTAs themselves: 1000 frames 79 us, with the planner's launch 87
 constexpr uint32_t AC1D_DIRECT = 1024;
 template <int INTERP>
-__global__ void __launch_bounds__(AC1D_THREADS, AC1D_PER_SM) ac1d_sparse_kernel(const AC1DArgs a)
+__global__ void __launch_bounds__(2 * AC1D_THREADS, 1) ac1d_sparse_kernel(const AC1DArgs a)
 {
     __shared__ unsigned long long s_off[AC1D_DIRECT + 1];
     __shared__ unsigned long long s_sums[32];
@@ -1133,6 +1130,8 @@ __global__ void __launch_bounds__(AC1D_THREADS, AC1D_PER_SM) ac1d_sparse_kernel(
     const uint32_t whole = (uint32_t)__cvta_generic_to_shared(h.whole), 
                    // without room every pair adds 0, at a word that exists
                    fixed = a.fixed ? (uint32_t)__cvta_generic_to_shared(h.fix_lo) : whole;
+    const uint32_t dev = (uint32_t)__cvta_generic_to_shared(h.dev_lo);
+    const uint32_t dev_bins = a.vecsize - INTERP;  // a pair's first bin below this: no bin wraps
     const uint32_t fix_bins = a.fixed ? a.size - 1 : 0u;  // a pair's first bin below this: both exist
     const float2 nz = make_float2(a.neg_zero, a.neg_zero);
     const float4 *__restrict__ P = nullptr;
@@ -1206,13 +1205,6 @@ __global__ void __launch_bounds__(AC1D_THREADS, AC1D_PER_SM) ac1d_sparse_kernel(
                             if (e ? rare[1] : rare[0])
                                 host_route_add(h.whole, a.size, a.counters, e ? bin[1] : bin[0], e ? v[1] : v[0]);
                     }
-                } else if (INTERP == 0) {
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        uint32_t iq;
-                        floor_small(fadd(q[e], 0.49999997f), iq);  // as above
-                        if (on[e]) device_route_add(a, h, iq, dmul(dmul((double)A.w, (double)bw[e]), a.mult));
-                    }
                 } else if (host) {
                     uint32_t at[2], bin[2], u[4];
                     float v[4];
@@ -1255,14 +1247,52 @@ __global__ void __launch_bounds__(AC1D_THREADS, AC1D_PER_SM) ac1d_sparse_kernel(
                         }
                     }
                 } else {
+                    constexpr int N = INTERP ? 2 : 1;  // bins of a pair
+                    uint32_t at[2], bin[2], u[2 * N];
+                    double x[2 * N];
+                    bool rare[2], c[2 * N], any = false;
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        uint32_t iq;
-                        const float fq = floor_small(q[e], iq);
-                        if (!on[e]) continue;
-                        const double sep = (double)fsub(q[e], fq), val = dmul((double)A.w, (double)bw[e]);
-                        device_route_add(a, h, iq, dmul(dmul(val, dsub(1.0, sep)), a.mult));
-                        device_route_add(a, h, iq + 1, dmul(dmul(val, sep), a.mult));
+                        const double val = dmul((double)A.w, (double)bw[e]);
+                        if (INTERP == 0) {
+                            floor_small(fadd(q[e], 0.49999997f), bin[e]);  // as above
+                            x[e] = dmul(val, a.mult);
+                        } else {
+                            const float fq = floor_small(q[e], bin[e]);
+                            const double sep = (double)fsub(q[e], fq);
+                            x[N * e] = dmul(dmul(val, dsub(1.0, sep)), a.mult);
+                            x[N * e + N - 1] = dmul(dmul(val, sep), a.mult);
+                        }
+                        const bool in = on[e] && bin[e] < dev_bins;
+                        at[e] = in ? dev + 4u * bin[e] : dev;  // off: adds 0
+                        bool ok = in;
+#pragma unroll
+                        for (int m = N * e; m < N * e + N; m++) {  // twice floor(x), x in [0, 2^31)
+                            const bool small = (uint32_t)__double2hiint(x[m]) < 0x41E00000u;
+                            u[m] = in && small ? 2u * (uint32_t)__double2loint(__dadd_rz(x[m], 4503599627370496.0)) : 0u;
+                            ok = ok && small;
+                        }
+                        rare[e] = on[e] && !ok;
+                    }
+#pragma unroll
+                    for (int m = 0; m < 2 * N; m++) {
+                        c[m] = shared_add32(at[m / N] + 4u * (m % N), u[m]) + u[m] < u[m];
+                        any = any || c[m];
+                    }
+                    if (any) {
+#pragma unroll
+                        for (int m = 0; m < 2 * N; m++)
+                            if (c[m]) shared_add32(at[m / N] + 4u * (m % N) + 4u * a.vecsize, 1u);
+                    }
+                    if (rare[0] || rare[1]) {
+#pragma unroll 1
+                        for (int m = 0; m < 2 * N; m++) {
+                            const bool second = m >= N, last = m % N != 0;
+                            const double y = second ? (last ? x[2 * N - 1] : x[N]) : (last ? x[N - 1] : x[0]);
+                            const uint32_t b = second ? bin[1] : bin[0];
+                            const bool small = b < dev_bins && (uint32_t)__double2hiint(y) < 0x41E00000u;
+                            if ((second ? rare[1] : rare[0]) && !small) device_route_add(a, h, b + last, y);
+                        }
                     }
                 }
             }
@@ -1487,7 +1517,9 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
     a.fix_top = (float)(2u << e);
     a.fix_mask = (1u << (22 - e)) - 1;
     const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(AC1D_PER_SM, (208u << 10) / std::max<size_t>(smem, 1)));
-    const int grid = ctx->sm_count * per_sm;
+    // shapes that leave one CTA an SM: twice the threads, unless the batch is short (3435
+    // bins, 1008 frames 92.7 -> 81.2 us; 4000 bins, 300 frames 27.8 -> 35.3)
+    const int grid = ctx->sm_count * per_sm, threads = per_sm == 1 && nframes > 512 ? 2 * AC1D_THREADS : AC1D_THREADS;
     const bool direct = nframes <= AC1D_DIRECT;
     unsigned long long *cost_off = (unsigned long long *)scratch;
     PlanHeader *head = (PlanHeader *)((char *)scratch + table_bytes);
@@ -1504,14 +1536,14 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
     a.mult = mult;
     if (!direct) {  // without the count check
         sparse_plan_kernel<<<PLAN_CTAS, PLAN_THREADS, 0, s>>>(d_off, nframes, a.walk.steps_max,
-                                                              (uint32_t)(grid * AC1D_THREADS / 32), cost_off, head,
+                                                              (uint32_t)(grid * threads / 32), cost_off, head,
                                                               a.walk.photons, nullptr, 0.0f, nullptr);
         IAC_LAUNCHED(ctx);
         IAC_CUDA(cudaGetLastError());
     }
     auto k = interp == 0 ? ac1d_sparse_kernel<0> : ac1d_sparse_kernel<1>;
     IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, AC1D_THREADS, smem, s>>>(a);
+    k<<<grid, threads, smem, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
     return IAC_OK;
