@@ -9,7 +9,7 @@ uint64 mesh (MeshSize 199), nearest/nearest with double mapping,
 Multiplicator 1000.  Seeded synthetic data of that shape.
 
 One step = the whole batch through the hot path: clear the half mesh, plan the
-work queue, bin every photon pair (persistent kernel), fold into the full mesh.
+walk, bin every photon pair (persistent kernel), fold into the full mesh.
 `value` times steps with inputs resident in HBM; `e2e` times the C-ABI host
 entry point with pinned host photon lists, the batches of a run accumulating
 into a device-resident mesh that is folded and read back once at the end of

@@ -155,7 +155,7 @@ uint64_t iac_full_mesh_words(uint32_t size_ab);
  *   d_half_mesh     accumulates the half mesh (ss >= 0) of the reference
  *                   kernel, uint64[iac_half_mesh_words(S)]; not cleared.
  * The call is asynchronous on `stream`.  It uses the context's scratch
- * (work-queue counters and the per-frame tile table). */
+ * (the batch's plan: a table of frame starts, a counter, per-frame flags). */
 iac_status iac_sparse_ac_batch(iac_ctx *ctx, const float *d_photons,
                                const uint64_t *d_frame_offsets, const float *d_rot9,
                                uint32_t nframes, const iac_sparse_params *params,

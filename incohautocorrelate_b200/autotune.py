@@ -1,4 +1,4 @@
-"""Autotuner of the persistent photon-pair kernel's work queue.
+"""Autotuner of the photon-pair kernel's launch shape.
 
 For each mesh edge it times the batched correlator over a grid of
 (tile_pairs, block_threads, ctas_per_sm, cache_hints) on a seeded workload of

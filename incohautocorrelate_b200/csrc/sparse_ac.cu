@@ -13,8 +13,8 @@
 // and walk the L partners i + d, so the partner loads of a step are 512
 // contiguous bytes and a step needs one load, no division and no ordering of
 // its two photons.  Frames are laid end to end by cost (units x (L + overhead))
-// and every warp of the launch takes an equal contiguous share of the batch's
-// cost: no work queue, no barrier between frames.  L comes from the batch's
+// and the warps of the launch take equal chunks of the batch's cost from one
+// counter: no queue of tiles, no barrier between frames.  L comes from the batch's
 // pair count, so that a single event still spreads over the GPU.
 //
 // Exactness.  All float operations are the reference's, in its order, as
@@ -1420,7 +1420,7 @@ static PairShape pair_shape(const iac_sparse_tuning &tun, int max_threads, int C
     return s;
 }
 
-// Work-queue memory of one batch: planner header, table of frame starts
+// Plan of one batch: planner header, table of frame starts
 // (nframes + 1), per-frame flags (nframes bytes).
 struct QueueMem {
     unsigned long long *cost_off;
@@ -1764,7 +1764,7 @@ static iac_status stage_and_bin(iac_ctx *ctx, const float *h_photons, const uint
         off_pos[k] = w;
         for (uint32_t f = cut[k]; f <= cut[k + 1]; f++) off[w++] = h_off[f] - h_off[cut[k]];
     }
-    {   // size the work-queue scratch for the largest chunk now: growing it
+    {   // size the plan's scratch for the largest chunk now: growing it
         // between chunk launches would synchronise the device
         void *t = nullptr;
         const size_t tb = ((sizeof(unsigned long long) * ((size_t)nframes + 1) + 127) / 128) * 128;
@@ -1867,8 +1867,8 @@ iac_status iac_sparse_ac_frames_host_to_device(iac_ctx *ctx, const float *h_phot
 // synchronisation and unbounded latency a cudaMalloc/cudaFree can cause, or a
 // host framework that hands out all device memory from its own pool and
 // forbids allocations behind its back.  iac_sparse_ac_batch grows a per-stream
-// scratch buffer on first use; this entry point instead keeps the same work
-// queue (tile table, queue counter, per-frame flags) in a fixed array of
+// scratch buffer on first use; this entry point instead keeps the same
+// plan (table of frame starts, chunk counter, per-frame flags) in a fixed array of
 // device memory that is part of the loaded library, so it never allocates.
 //
 // The array's name in host code only stands in for the symbol; the kernels
@@ -1880,10 +1880,10 @@ iac_status iac_sparse_ac_frames_host_to_device(iac_ctx *ctx, const float *h_phot
 // context's device state), so the kept address is never stale while the
 // context is usable.  The array is shared by every call on the device and
 // keeps the previous call's contents: the planner kernel rewrites the whole
-// tile table and resets the queue counter before the pair kernel reads them,
+// table and resets the counter before the pair kernel reads them,
 // so nothing has to be cleared from the host, but two calls running on the
 // GPU at the same time (e.g. on two streams) would overwrite each other's
-// queue.
+// plan.
 // ---------------------------------------------------------------------------
 namespace iac {
 
