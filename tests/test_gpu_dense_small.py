@@ -74,3 +74,21 @@ def test_ac1d_small_values(ctx, oracle_lib, rng, interp, ny, nx, size, cut):
             out = _dev(np.zeros(want.size, np.int64))
             ctx.ac1d_cq(_dev(I), _dev(k), npix, sh, interp, mult, out)
             np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=f"{name} {wrap}")
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+@pytest.mark.parametrize("edge", [25, 45, 61, 81, 121])
+def test_cq_small_window_sizes(ctx, oracle_lib, rng, interp, edge):
+    """Meshes whose tile windows fill a part of the shared-memory window, just
+    fit it, or exceed it in some or all tile pairs."""
+    o = oracle_lib
+    ny, nx = 37, 44
+    _, km, mq = small_detector(ny, nx, 6e-4)
+    I = rng.uniform(0.05, 1.5, ny * nx).astype(np.float32)
+    s = o.small_cq_mesh_shape(mq, edge)
+    want = np.zeros(s.size_ab * s.size_ab * s.size_c, np.uint64)
+    o.lib().iaco_cq_small(o.p(I), o.p(km), ny * nx, s, interp, 123457.0, 0, ny * nx, o.p(want))
+    for fast in (0, nx):
+        out = _dev(np.zeros(want.size, np.int64))
+        ctx.cq_small(_dev(I), _dev(km), ny * nx, to_capi_shape(s), interp, 123457.0, out, fast_size=fast)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=str(fast))
