@@ -40,12 +40,15 @@
 namespace iac {
 
 constexpr int DTILE = 256;        // pixels per tile == threads per CTA
-// Shared-memory window: split 64-bit counters, 32 KB, six CTAs an SM.  A tile pair
-// whose q range is larger adds every pair, and its mirror, in L2 instead.  2048
-// against 4096 words: nearest 120 x 150, 199-edge mesh 1.80 -> 0.55 ms; linear
-// 240 x 280, 253-edge mesh 128 -> 11.1 ms, 200 x 240 at 199 46.2 -> 5.9 ms, 120 x 150
-// at 199 14.1 -> 11.5 ms; maps whose windows already fitted the same within 0.1 %.
-constexpr int WINDOW_WORDS = 4096;
+// Shared-memory window: split 64-bit counters.  A tile pair whose q range is larger
+// adds every pair, and its mirror, in L2 instead, which costs far more than the
+// window's memory: as many words as six (linear: four) CTAs an SM leave room for.
+// 2048, 4096 and 5440 words: linear 240 x 280, 253-edge mesh 128, 11.1 and 11.1 ms,
+// 160 x 180 at 253 27.9 -> 15.7 from 4096 to 5440, 120 x 150 at 199 14.1, 11.5 and 2.7;
+// nearest 120 x 150, 199-edge mesh 1.80 -> 0.55 ms from 2048 to 4096, but 300 x 350 at
+// 253 6.34 -> 6.57 from 4096 to 5440, where only four CTAs fit.
+template <int INTERP>
+constexpr int WINDOW_WORDS = INTERP ? 5440 : 4096;
 
 struct DenseArgs {
     const float *__restrict__ I;
@@ -218,6 +221,7 @@ __device__ __forceinline__ void global_put_pair(const DenseArgs &a, int fs, int 
     }
 }
 
+template <int INTERP>
 __device__ __forceinline__ void put(const DenseArgs &a, const Window &w, uint32_t *win,
                                     int fs, int ms, int ss, unsigned long long v)
 {
@@ -225,7 +229,7 @@ __device__ __forceinline__ void put(const DenseArgs &a, const Window &w, uint32_
     const int x = fs - w.lo[0], y = ms - w.lo[1], z = ss - w.lo[2];
     if (w.on && (unsigned)x < (unsigned)w.dim[0] && (unsigned)y < (unsigned)w.dim[1] &&
         (unsigned)z < (unsigned)w.dim[2])
-        shared_add_u64_split(win, win + WINDOW_WORDS, x + w.dim[0] * (y + w.dim[1] * z), v);
+        shared_add_u64_split(win, win + WINDOW_WORDS<INTERP>, x + w.dim[0] * (y + w.dim[1] * z), v);
     else
         global_put_pair(a, fs, ms, ss, v);
 }
@@ -288,11 +292,11 @@ __device__ __forceinline__ void cq_pairs(const DenseArgs &a, const Window &w, ui
         if (!have || f != cur_f || m != cur_m || s != cur_s) {
             if (have) {
                 if (INTERP == 0) {
-                    put(a, w, win, cur_f, cur_m, cur_s, acc[0]);
+                    put<INTERP>(a, w, win, cur_f, cur_m, cur_s, acc[0]);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 8; c++)
-                        put(a, w, win, cur_f + (c >> 2), cur_m + ((c >> 1) & 1), cur_s + (c & 1), acc[c]);
+                        put<INTERP>(a, w, win, cur_f + (c >> 2), cur_m + ((c >> 1) & 1), cur_s + (c & 1), acc[c]);
                 }
             }
             have = true;
@@ -318,11 +322,11 @@ __device__ __forceinline__ void cq_pairs(const DenseArgs &a, const Window &w, ui
     }
     if (have) {
         if (INTERP == 0) {
-            put(a, w, win, cur_f, cur_m, cur_s, acc[0]);
+            put<INTERP>(a, w, win, cur_f, cur_m, cur_s, acc[0]);
         } else {
 #pragma unroll
             for (int c = 0; c < 8; c++)
-                put(a, w, win, cur_f + (c >> 2), cur_m + ((c >> 1) & 1), cur_s + (c & 1), acc[c]);
+                put<INTERP>(a, w, win, cur_f + (c >> 2), cur_m + ((c >> 1) & 1), cur_s + (c & 1), acc[c]);
         }
     }
 }
@@ -363,7 +367,7 @@ __device__ __forceinline__ void cq_pairs_nn(const DenseArgs &a, const Window &w,
         const int s = round_half_away(axis<KC>(qx, qy, qz, 0));
         const int key = f + m * 1024 + s * 1048576;
         if (key != cur) {
-            if (cur != NONE) put(a, w, win, cf + a.cab, cm + a.cab, cs + a.cc, acc);
+            if (cur != NONE) put<0>(a, w, win, cf + a.cab, cm + a.cab, cs + a.cc, acc);
             cur = key;
             cf = f;
             cm = m;
@@ -372,7 +376,7 @@ __device__ __forceinline__ void cq_pairs_nn(const DenseArgs &a, const Window &w,
         }
         acc += MINT ? scaled_floor_normal(pv, a.mult_int) : d2u64(dmul((double)pv, a.mult));
     }
-    if (cur != NONE) put(a, w, win, cf + a.cab, cm + a.cab, cs + a.cc, acc);
+    if (cur != NONE) put<0>(a, w, win, cf + a.cab, cm + a.cab, cs + a.cc, acc);
 }
 
 
@@ -410,14 +414,14 @@ __device__ __forceinline__ void cq_pairs_win(const DenseArgs &a, const Window &w
         const int key = base + f + D0 * m + D01 * sz;
         const unsigned long long v = MINT ? scaled_floor_normal(pv, a.mult_int) : d2u64(dmul((double)pv, a.mult));
         const bool brk = ok && (!on || key != cur);  // a new run starts at this pair
-        if (brk && on) shared_add_u64_split(win, win + WINDOW_WORDS, (uint32_t)cur, acc);
+        if (brk && on) shared_add_u64_split(win, win + WINDOW_WORDS<0>, (uint32_t)cur, acc);
         const bool inwin = (unsigned)key < (unsigned)words;
         if (brk && !inwin) global_put_pair(a, f + a.cab, m + a.cab, sz + a.cc, v);
         acc = brk ? (inwin ? v : 0ull) : (ok ? acc + v : acc);
         cur = brk ? key : cur;
         on = brk ? inwin : on;
     }
-    if (on) shared_add_u64_split(win, win + WINDOW_WORDS, (uint32_t)cur, acc);
+    if (on) shared_add_u64_split(win, win + WINDOW_WORDS<0>, (uint32_t)cur, acc);
 }
 
 // ---- two consecutive staged pixels per step, FP32 work as f32x2 pairs ----
@@ -451,7 +455,7 @@ __device__ __forceinline__ void win_step(const DenseArgs &a, uint32_t *win, int 
     const int k = ok ? key : cur;
     const unsigned long long v = scaled_floor_small(ok ? pv : 0.0f, a.mult_int);
     const bool brk = k != cur;
-    if (brk) shared_add_u64_split(win, win + WINDOW_WORDS, (uint32_t)cur, acc);  // acc may be 0: adds nothing
+    if (brk) shared_add_u64_split(win, win + WINDOW_WORDS<0>, (uint32_t)cur, acc);  // acc may be 0: adds nothing
     acc = (brk ? 0ull : acc) + v;
     cur = k;
 }
@@ -496,7 +500,7 @@ __device__ __forceinline__ void cq_pairs_win2(const DenseArgs &a, const Window &
     if (j0 & 1) step(jp++, false);
 #pragma unroll 2
     for (; jp < DTILE / 2; jp++) step(jp, true);
-    if (acc) shared_add_u64_split(win, win + WINDOW_WORDS, (uint32_t)cur, acc);
+    if (acc) shared_add_u64_split(win, win + WINDOW_WORDS<0>, (uint32_t)cur, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -530,7 +534,7 @@ __device__ __forceinline__ void window_add_halves(uint32_t win, int at, uint32_t
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p red.shared.add.u32 [%1], %2;\n\t"
         "@p red.shared.add.u32 [%1+%4], %3;\n\t}" ::"r"((int)on),
-        "r"(win + 4u * (uint32_t)at), "r"(acc & 0xffffu), "r"(acc >> 16), "n"(4 * WINDOW_WORDS)
+        "r"(win + 4u * (uint32_t)at), "r"(acc & 0xffffu), "r"(acc >> 16), "n"(4 * WINDOW_WORDS<0>)
         : "memory");
 }
 
@@ -612,7 +616,7 @@ __device__ __forceinline__ void cq_pairs_small_linear(const DenseArgs &a, const 
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             if (old[c] + acc[c] < old[c])  // rare: the carry out of the low word
-                asm volatile("red.shared.add.u32 [%0+%1], 1;" ::"r"(at(c)), "n"(4 * WINDOW_WORDS) : "memory");
+                asm volatile("red.shared.add.u32 [%0+%1], 1;" ::"r"(at(c)), "n"(4 * WINDOW_WORDS<1>) : "memory");
             acc[c] = 0;
         }
     };
@@ -677,7 +681,7 @@ template <int INTERP, int KA, int KB, int KC>
 __global__ void __launch_bounds__(DTILE, INTERP ? 4 : 6) cq_small_kernel(const DenseArgs a)
 {
     __shared__ float4 sq[DTILE];
-    __shared__ uint32_t win[2 * WINDOW_WORDS];  // split 64-bit counters: low words, then high words
+    __shared__ uint32_t win[2 * WINDOW_WORDS<INTERP>];  // split 64-bit counters: low words, then high words
     __shared__ unsigned long long s_pair;
     __shared__ unsigned long long s_self[DTILE / 32];
     const uint32_t T = a.ntiles;
@@ -708,12 +712,12 @@ __global__ void __launch_bounds__(DTILE, INTERP ? 4 : 6) cq_small_kernel(const D
                 const float h = (ax[d] == 0 ? hi3[0] : ax[d] == 1 ? hi3[1] : hi3[2]) * a.vpdq;
                 w.lo[d] = (int)floorf(l) - 1 + cen[d];
                 w.dim[d] = (int)ceilf(h) + 2 + cen[d] - w.lo[d] + (INTERP ? 1 : 0);
-                ok &= w.dim[d] >= 1 && w.dim[d] <= WINDOW_WORDS;
-                words *= max(1, min(w.dim[d], WINDOW_WORDS + 1));
+                ok &= w.dim[d] >= 1 && w.dim[d] <= WINDOW_WORDS<INTERP>;
+                words *= max(1, min(w.dim[d], WINDOW_WORDS<INTERP> + 1));
             }
-            w.on = ok && words <= WINDOW_WORDS;
+            w.on = ok && words <= WINDOW_WORDS<INTERP>;
             if (w.on)
-                for (int i = threadIdx.x; i < words; i += DTILE) win[i] = win[WINDOW_WORDS + i] = 0u;
+                for (int i = threadIdx.x; i < words; i += DTILE) win[i] = win[WINDOW_WORDS<INTERP> + i] = 0u;
         }
         const bool small = KA >= 0 && w.on && (INTERP || a.mult_f != 0.0f) && small_values(a, p0, p1, q0, q1);
         // integer Multiplicator and every product of the two tiles below 2^23
@@ -812,8 +816,8 @@ __global__ void __launch_bounds__(DTILE, INTERP ? 4 : 6) cq_small_kernel(const D
             const int words = w.dim[0] * w.dim[1] * w.dim[2];
             for (int i = threadIdx.x; i < words; i += DTILE) {
                 const unsigned long long v =
-                    small && !INTERP ? win[i] + ((unsigned long long)win[WINDOW_WORDS + i] << 16)
-                                     : split_word(win, win + WINDOW_WORDS, i);
+                    small && !INTERP ? win[i] + ((unsigned long long)win[WINDOW_WORDS<INTERP> + i] << 16)
+                                     : split_word(win, win + WINDOW_WORDS<INTERP>, i);
                 if (!v) continue;
                 const int x = i % w.dim[0], y = (i / w.dim[0]) % w.dim[1], z = i / (w.dim[0] * w.dim[1]);
                 global_put_pair(a, x + w.lo[0], y + w.lo[1], z + w.lo[2], v);
