@@ -197,8 +197,12 @@ __global__ void __launch_bounds__(MERGE_THREADS, 1) merge_kernel(const MergeArgs
                     }
                     const bool in = i[0] < ab - 1 && i[1] < ab - 1 && i[2] < ab - 1;
                     if (on && !in) merge_any<1>(a, vin, w, q[0], q[1], q[2]);
-                    const double base = on && in ? dmul(dmul(vin, a.mult), w) : 0.0;
-                    const unsigned long long at = on && in ? i[0] + ab * (i[1] + ab * (unsigned long long)i[2]) : 0ull;
+                    const bool add = on && in;
+                    if (!add)
+#pragma unroll
+                        for (int k = 0; k < 3; k++) s[k] = c[k] = 0.0;  // NaN where q is not finite: 0 * NaN is no 0
+                    const double base = add ? dmul(dmul(vin, a.mult), w) : 0.0;
+                    const unsigned long long at = add ? i[0] + ab * (i[1] + ab * (unsigned long long)i[2]) : 0ull;
                     // even lanes add a voxel's lower word while odd lanes add the upper one of
                     // the same voxel: first the even lanes' voxels, then the odd lanes'
                     const unsigned long long there = __shfl_xor_sync(0xffffffffu, at, 1);
