@@ -710,12 +710,16 @@ __global__ void __launch_bounds__(DTILE, INTERP ? 4 : 6) cq_small_kernel(const D
             for (int d = 0; d < 3; d++) {
                 const float l = (ax[d] == 0 ? lo3[0] : ax[d] == 1 ? lo3[1] : lo3[2]) * a.vpdq;
                 const float h = (ax[d] == 0 ? hi3[0] : ax[d] == 1 ? hi3[1] : hi3[2]) * a.vpdq;
-                w.lo[d] = (int)floorf(l) - 1 + cen[d];
-                w.dim[d] = (int)ceilf(h) + 2 + cen[d] - w.lo[d] + (INTERP ? 1 : 0);
-                ok &= w.dim[d] >= 1 && w.dim[d] <= WINDOW_WORDS<INTERP>;
-                words *= max(1, min(w.dim[d], WINDOW_WORDS<INTERP> + 1));
+                // coordinates below 2^22, where their roundings are exact and nothing here
+                // overflows; false for a range that is not finite
+                ok = ok && l > -4194304.0f && h < 4194304.0f && h - l <= (float)WINDOW_WORDS<INTERP>;
+                w.lo[d] = ok ? (int)floorf(l) - 1 + cen[d] : 0;
+                w.dim[d] = ok ? (int)ceilf(h) + 2 + cen[d] - w.lo[d] + (INTERP ? 1 : 0) : 0;
+                ok = ok && w.dim[d] >= 1 && w.dim[d] <= WINDOW_WORDS<INTERP>;
+                if (ok) words *= w.dim[d];  // at most WINDOW_WORDS^2 here
+                ok = ok && words <= WINDOW_WORDS<INTERP>;
             }
-            w.on = ok && words <= WINDOW_WORDS<INTERP>;
+            w.on = ok;
             if (w.on)
                 for (int i = threadIdx.x; i < words; i += DTILE) win[i] = win[WINDOW_WORDS<INTERP> + i] = 0u;
         }

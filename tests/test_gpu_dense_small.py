@@ -92,3 +92,36 @@ def test_cq_small_window_sizes(ctx, oracle_lib, rng, interp, edge):
         out = _dev(np.zeros(want.size, np.int64))
         ctx.cq_small(_dev(I), _dev(km), ny * nx, to_capi_shape(s), interp, 123457.0, out, fast_size=fast)
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=str(fast))
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+@pytest.mark.parametrize("case", ["far pixels", "window product past 2^31", "coordinates past 2^22"])
+def test_cq_window_past_the_integers(ctx, oracle_lib, rng, interp, case):
+    """Tile pairs whose q range the window's integers cannot hold: pixels whose k is
+    finite but far off, a window of 1 480 voxels on each axis, and a small window at
+    voxel 2^23.  What lies outside the mesh is skipped, the rest is the oracle's."""
+    o = oracle_lib
+    npix = 3 * 256 + 17
+    s = o.small_cq_mesh_shape(np.array([1.0, 0.9, 0.4], np.float32), 41)
+    k = rng.uniform(0.0, 0.01, (npix, 3)).astype(np.float32)
+    s.voxel_per_dq, s.max_q = 1500, np.float32(4.0)
+    if case == "far pixels":
+        k[5::64] = np.float32(1e18)
+        k[37::64] = np.float32(-1e18)
+    elif case == "window product past 2^31":
+        s.voxel_per_dq = 740
+        k = rng.uniform(0.0, 1.0, (npix, 3)).astype(np.float32)
+        k[::5] = k[0] + rng.uniform(0.0, 0.01, (len(k[::5]), 3)).astype(np.float32)
+    else:
+        s.voxel_per_dq = 1 << 23
+        k = rng.uniform(0.0, 1e-6, (npix, 3)).astype(np.float32)
+        k[256:512, 0] += np.float32(1.0)
+    I = rng.uniform(0.05, 1.5, npix).astype(np.float32)
+    want = np.zeros(s.size_ab * s.size_ab * s.size_c, np.uint64)
+    k = np.ascontiguousarray(k.reshape(-1))
+    o.lib().iaco_cq_small(o.p(I), o.p(k), npix, s, interp, 1000.0, 0, npix, o.p(want))
+    assert want.any()
+    out = _dev(np.zeros(want.size, np.int64))
+    ctx.cq_small(_dev(I), _dev(k), npix, to_capi_shape(s), interp, 1000.0, out)
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want)
+    ctx.check()
