@@ -565,8 +565,8 @@ __device__ __forceinline__ void cq_pairs_small(const DenseArgs &a, const Window 
         if (CHECK) {
             const float2 nz = dup(a.neg_zero);
             const float2 s = f2add(f2add(f2fma(qx, qx, nz), f2fma(qy, qy, nz)), f2fma(qz, qz, nz));
-            ok0 = ok0 && s.x <= a.maxq2;
-            ok1 = s.y <= a.maxq2;
+            ok0 = ok0 && !(s.x > a.maxq2);  // a MaxQ that is no number bounds nothing
+            ok1 = !(s.y > a.maxq2);
         }
         const float2 vp = dup(a.vpdq);
         qx = f2mul(qx, vp);
@@ -631,7 +631,7 @@ __device__ __forceinline__ void cq_pairs_small_linear(const DenseArgs &a, const 
         const float4 b = sq[j];
         float pv = fmul(Ia, b.w);
         float qx = fsub(k0, b.x), qy = fsub(k1, b.y), qz = fsub(k2, b.z);
-        const bool ok = !CHECK || fadd(fadd(fmul(qx, qx), fmul(qy, qy)), fmul(qz, qz)) <= a.maxq2;
+        const bool ok = !CHECK || !(fadd(fadd(fmul(qx, qx), fmul(qy, qy)), fmul(qz, qz)) > a.maxq2);
         qx = fmul(qx, a.vpdq);
         qy = fmul(qy, a.vpdq);
         qz = fmul(qz, a.vpdq);

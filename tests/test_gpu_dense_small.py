@@ -125,3 +125,20 @@ def test_cq_window_past_the_integers(ctx, oracle_lib, rng, interp, case):
     ctx.cq_small(_dev(I), _dev(k), npix, to_capi_shape(s), interp, 1000.0, out)
     np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want)
     ctx.check()
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+def test_cq_maxq_that_bounds_nothing(ctx, oracle_lib, rng, interp):
+    """A MaxQ that is no number or infinite: every pair counts, as |q| > MaxQ is false."""
+    o = oracle_lib
+    _, km, mq = small_detector(17, 31, 6e-4)
+    I = rng.uniform(0.05, 1.5, 17 * 31).astype(np.float32)
+    s = o.small_cq_mesh_shape(mq, 41)
+    for s.max_q in (np.nan, np.inf):
+        want = np.zeros(s.size_ab * s.size_ab * s.size_c, np.uint64)
+        o.lib().iaco_cq_small(o.p(I), o.p(km), I.size, s, interp, 123457.0, 0, I.size, o.p(want))
+        assert want.any()
+        out = _dev(np.zeros(want.size, np.int64))
+        ctx.cq_small(_dev(I), _dev(km), I.size, to_capi_shape(s), interp, 123457.0, out, fast_size=31)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want)
+    ctx.check()
