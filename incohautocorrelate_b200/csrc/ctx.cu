@@ -144,7 +144,9 @@ iac_status iac_ctx_create(int device, iac_ctx **out)
     cudaMemset(c->d_counters, 0, sizeof(DeviceCounters));
     cudaDeviceSynchronize();
     // device address of the allocation-free entry point's fixed scratch array
-    const iac_status st = static_scratch_setup(c);
+    iac_status st = static_scratch_setup(c);
+    if (st == IAC_OK) st = pair_kernel_limits();
+    if (st == IAC_OK) st = dense_kernel_limits();
     if (st != IAC_OK) {
         cudaFree(c->d_counters);
         delete c;

@@ -1184,6 +1184,18 @@ __global__ void __launch_bounds__(DTILE) ac1d_rows_kernel(const DenseArgs a, con
         if (hist[i]) atomicAdd(&a.out[i], hist[i]);
 }
 
+constexpr uint32_t AC1D_MAX_SIZE = 24576;  // bins of a shared-memory histogram of 64-bit words
+
+iac_status dense_kernel_limits()
+{
+    constexpr int hist = (int)(sizeof(unsigned long long) * AC1D_MAX_SIZE);
+    for (auto k : {ac1d_cq_kernel<0>, ac1d_cq_kernel<1>})
+        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, hist));
+    for (auto k : {ac1d_rows_kernel<0>, ac1d_rows_kernel<1>})
+        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, hist));
+    return IAC_OK;
+}
+
 static float sqrt_threshold(float m)
 {
     if (!(m >= 0.0f) || std::isinf(m)) return m;
@@ -1330,7 +1342,8 @@ iac_status iac_ac1d_cq_part(iac_ctx *ctx, const float *d_I, const float *d_kmap,
     IAC_REQUIRE(nparts >= 1 && part < nparts, "iac_ac1d_cq_part: part %u of %u", part, nparts);
     IAC_REQUIRE(interp == 0 || interp == 1, "interpolation must be 0 or 1");
     IAC_REQUIRE(npix > 0 && npix < (1ull << 32), "iac_ac1d_cq: pixel count out of range");
-    IAC_REQUIRE(sh->size >= 3 && sh->size <= 24576, "AC1D size %u out of range [3, 24576]", sh->size);
+    IAC_REQUIRE(sh->size >= 3 && sh->size <= AC1D_MAX_SIZE, "AC1D size %u out of range [3, %u]", sh->size,
+                AC1D_MAX_SIZE);
     IAC_REQUIRE(sh->dq_per_step > 0 && (double)sh->max_q / sh->dq_per_step < 4194304.0,
                 "iac_ac1d_cq: MaxQ / dq must be below 2^22 (dq %g, MaxQ %g)", (double)sh->dq_per_step,
                 (double)sh->max_q);
@@ -1353,7 +1366,6 @@ iac_status iac_ac1d_cq_part(iac_ctx *ctx, const float *d_I, const float *d_kmap,
                  (double)sh->max_q / sh->dq_per_step * 1.000001 < (double)sh->size - 1.0;
     const size_t smem = sizeof(unsigned long long) * sh->size;
     auto k = interp == 0 ? ac1d_cq_kernel<0> : ac1d_cq_kernel<1>;
-    IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<ctx->sm_count * 8, DTILE, smem, as_stream(stream)>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
@@ -1417,7 +1429,8 @@ iac_status iac_ac1d_cq_rows(iac_ctx *ctx, const float *d_I, const float *d_kmap,
     IAC_REQUIRE(interp == 0 || interp == 1, "interpolation must be 0 or 1");
     IAC_REQUIRE(npix > 0 && npix < (1ull << 32), "iac_ac1d_cq_rows: pixel count out of range");
     IAC_REQUIRE(nrows >= 1, "iac_ac1d_cq_rows: no rows");
-    IAC_REQUIRE(sh->size >= 3 && sh->size <= 24576, "AC1D size %u out of range [3, 24576]", sh->size);
+    IAC_REQUIRE(sh->size >= 3 && sh->size <= AC1D_MAX_SIZE, "AC1D size %u out of range [3, %u]", sh->size,
+                AC1D_MAX_SIZE);
     IAC_REQUIRE(mult > 0, "multiplicator must be positive");
     DeviceGuard g(ctx->device);
     DenseArgs a{};
@@ -1439,7 +1452,6 @@ iac_status iac_ac1d_cq_rows(iac_ctx *ctx, const float *d_I, const float *d_kmap,
     IAC_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), s));
     const size_t smem = sizeof(unsigned long long) * sh->size;
     auto k = interp == 0 ? ac1d_rows_kernel<0> : ac1d_rows_kernel<1>;
-    IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<ctx->sm_count * 4, DTILE, smem, s>>>(a, d_rows, nrows);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());

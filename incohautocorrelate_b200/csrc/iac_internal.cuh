@@ -150,6 +150,13 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // it in the context.
 iac_status static_scratch_setup(iac_ctx *ctx);
 
+// Dynamic shared memory that the kernels whose need varies with a call's shape may
+// take (sparse_ac.cu, dense_pairs.cu), set with the context's device current when a
+// context is created.  The limit belongs to the kernel, and host threads share the
+// kernels: a launch that set its own size could find it lowered by another's.
+iac_status pair_kernel_limits();
+iac_status dense_kernel_limits();
+
 // Scratch slot `slot` of `stream`, grown to at least `bytes`.
 inline iac_status stream_scratch(iac_ctx *ctx, void *stream, int slot, size_t bytes, void **out)
 {

@@ -1335,11 +1335,25 @@ __global__ void ac1d_uw_finish_kernel(const unsigned long long *__restrict__ dev
 
 typedef void (*PairKernel)(SparseArgs);
 
+// dynamic shared memory at most: the boxes of an SM's CTAs, and the histograms of an AC1D CTA
+constexpr size_t PAIR_BOX_BYTES = 184u << 10, AC1D_HIST_BYTES = 216u << 10;
+
 static PairKernel pick_kernel(int dmap, int i1, int i2)
 {
     if (!dmap) return i2 ? sparse_pairs_kernel<0, 0, 1> : sparse_pairs_kernel<0, 0, 0>;
     if (i1 == 0) return i2 ? sparse_pairs_kernel<1, 0, 1> : sparse_pairs_kernel<1, 0, 0>;
     return i2 ? sparse_pairs_kernel<1, 1, 1> : sparse_pairs_kernel<1, 1, 0>;
+}
+
+iac_status pair_kernel_limits()
+{
+    const PairKernel pair[] = {sparse_pairs_kernel<0, 0, 0>, sparse_pairs_kernel<0, 0, 1>, sparse_pairs_kernel<1, 0, 0>,
+                               sparse_pairs_kernel<1, 0, 1>, sparse_pairs_kernel<1, 1, 0>, sparse_pairs_kernel<1, 1, 1>};
+    for (PairKernel k : pair)
+        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_BOX_BYTES));
+    for (auto k : {ac1d_sparse_kernel<0>, ac1d_sparse_kernel<1>})
+        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AC1D_HIST_BYTES));
+    return IAC_OK;
 }
 
 // Explicit settings win; otherwise the autotuner row of the nearest mesh edge;
@@ -1414,7 +1428,7 @@ static PairShape pair_shape(const iac_sparse_tuning &tun, int max_threads, int C
     PairShape s;
     s.ctas = (total + max_threads - 1) / max_threads;
     s.threads = std::max(32, std::min(max_threads, (total / s.ctas + 31) / 32 * 32));
-    const int budget = (184 << 10) / s.ctas;
+    const int budget = (int)PAIR_BOX_BYTES / s.ctas;
     s.box_max = std::min(BOX_R_MAX, C);
     while (s.box_max >= 0 && 4 * (s.box_max + 1) * (2 * s.box_max + 1) * (2 * s.box_max + 1) > budget) s.box_max--;
     return s;
@@ -1485,8 +1499,6 @@ static iac_status launch_pair_batch(iac_ctx *ctx, const float *d_photons, const 
     }
     const size_t box_bytes = sizeof(uint32_t) * (size_t)(sh.box_max + 1) * (2 * sh.box_max + 1) * (2 * sh.box_max + 1);
     const PairKernel k = pick_kernel(p->double_map, p->interp_first, p->interp_second);
-    if (box_bytes > (40u << 10))
-        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)box_bytes));
     k<<<grid, sh.threads, box_bytes, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
@@ -1508,7 +1520,7 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
     // the fixed-point histogram where two CTAs an SM (one, for large shapes) still fit
     const size_t plain = sizeof(unsigned long long) * ((size_t)b.vecsize + 2 * (size_t)b.size),
                  more = sizeof(unsigned long long) * b.size;
-    a.fixed = interp == 1 && b.size > 1 && plain + more <= (216u << 10);
+    a.fixed = interp == 1 && b.size > 1 && plain + more <= AC1D_HIST_BYTES;
     const size_t smem = plain + (a.fixed ? more : 0);
     // |q| / dq from 2^e on is a multiple of 2^(e - 23): with 2^(e + 1) for the top, the
     // counts' values are too; the first 2^e bins, 1/32 of them, see few of the pairs
@@ -1542,7 +1554,6 @@ static iac_status launch_ac1d_batch(iac_ctx *ctx, const float *d_photons, const 
         IAC_CUDA(cudaGetLastError());
     }
     auto k = interp == 0 ? ac1d_sparse_kernel<0> : ac1d_sparse_kernel<1>;
-    IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<grid, threads, smem, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
