@@ -318,15 +318,10 @@ def measured_bf16_tflops():
     return 1400.0, "fallback (1.4 PFLOP/s sustained)"
 
 
-def pair_box_radius(C, ctas_per_sm):
+def pair_box_radius(C):
     """Half-width of the pair kernel's shared-memory box around q = 0 for a
-    large batch (the library's rule: 22, shrunk until the boxes of an SM's CTAs
-    of (R + 1)(2R + 1)^2 32-bit words fit in 184 KB, at most the mesh centre)."""
-    budget = (184 << 10) // max(1, ctas_per_sm)
-    r = min(22, C)
-    while r > 0 and 4 * (r + 1) * (2 * r + 1) ** 2 > budget:
-        r -= 1
-    return r
+    large batch (the library's rule: 22, at most the mesh centre)."""
+    return min(22, C)
 
 
 def box_value_share(half, S, R, self_sum):
@@ -462,8 +457,7 @@ def run_ours(args):
     updates = pairs - int(len(ph_h))
     upd_rate = updates / (ms_kernel * 1e-3)
     tun = ctx.sparse_tuning(S)
-    # the threads of a setting run in as few CTAs of up to 1 024 as hold them
-    R = pair_box_radius((S - 1) // 2, -(-tun["block_threads"] * tun["ctas_per_sm"] // 1024))
+    R = pair_box_radius((S - 1) // 2)
     self_sum = 1000.0 * float((ph_h[:, 3].astype(np.float64) ** 2).sum())
     share = box_value_share(half, S, R, self_sum) if R > 0 else 0.0
 

@@ -219,7 +219,7 @@ iac_status iac_sparse_ac_batch_static(iac_ctx *ctx, const float *d_photons,
 typedef struct {
     uint32_t tile_pairs;      /* pairs a warp walks in one unit, at most 1 024 (32 lanes x 32 partners) */
     uint32_t block_threads;   /* block_threads x ctas_per_sm threads run per SM, */
-    uint32_t ctas_per_sm;     /* in as few CTAs (of up to 1 024) as hold them    */
+    uint32_t ctas_per_sm;     /* as one CTA, up to the 1 024 (512) it can have   */
     uint32_t cache_hints;     /* L2 policy: 1 = keep the mesh resident (evict-last
                                  atomics, evict-first photon loads), 2 = none  */
 } iac_sparse_tuning;

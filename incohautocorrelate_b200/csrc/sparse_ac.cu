@@ -415,7 +415,7 @@ __device__ __forceinline__ void chunk_steps(uint32_t n, uint32_t i, uint32_t c, 
 // Half-width R of the shared-memory box of voxels around q = 0 (ss <= R,
 // |fs - C| <= R, |ms - C| <= R) that each CTA of the pair kernel accumulates
 // privately, by the batch's distinct pairs: none below BOX_PAIRS_SMALL,
-// BOX_R_SMALL below BOX_PAIRS_LARGE, else what the launch has room for.  L2
+// BOX_R_SMALL below BOX_PAIRS_LARGE, else BOX_R_MAX (BOX_R_HEAVY).  L2
 // takes scattered adds at about 2e11 per second, one request each, whatever
 // their width, so every add that stays in the box counts: in a 201^3 mesh of
 // the rotated workload R = 22 keeps 32 % of them, R = 10 9 %.  100 000 frames
@@ -425,6 +425,7 @@ __device__ __forceinline__ void chunk_steps(uint32_t n, uint32_t i, uint32_t c, 
 // 148 at 22; 3 000 frames 273, 251 and 229; 300 frames 103, 104 and 118.
 constexpr int BOX_R_MAX = 22;    // 23 x 45 x 45 words: 186 KB
 constexpr int BOX_R_SMALL = 10;
+constexpr int BOX_R_HEAVY = 17;  // the most where the first level is linear
 constexpr unsigned long long BOX_PAIRS_SMALL = 1000000ull, BOX_PAIRS_LARGE = 20000000ull;
 
 struct SparseArgs {
@@ -444,7 +445,7 @@ struct SparseArgs {
     int check_here;   // no planner ran: the CTA checks its frames itself
     int fast_ok;      // MaxQ is finite
     int cache_hints;  // 1: mesh atomics evict-last, photon loads evict-first in L2; else no preference
-    int box_max;      // largest half-width of the shared-memory box that the launch has room for
+    int box_max;      // half-width of the largest shared-memory box
     // set inside the kernel
     uint64_t mesh_policy, photon_policy;
     float box_lim;    // |rotated component| below this rounds into the box (box_r + 0.5; 0: no box)
@@ -861,8 +862,7 @@ __global__ void __launch_bounds__(pair_threads(DMAP, I1, I2), 1) sparse_pairs_ke
     if (FAST && a.fast_ok && a.check_here) {  // the planner's check, for the frames of this CTA
         for (uint32_t f = threadIdx.x; f < a.walk.nframes; f += nthr) s_flags[f] = 1u;
         __syncthreads();
-        for (uint32_t f = 0; f < a.walk.nframes; f++) {
-            if (off[f + 1] <= share.x0 || off[f] >= share.x1) continue;
+        for (uint32_t f = warp_find_frame(off, a.walk.nframes, share.x0); f < a.walk.nframes && off[f] < share.x1; f++) {
             const uint64_t b = a.walk.offsets[f], e = a.walk.offsets[f + 1];
             uint32_t m = threadIdx.x >= 3 || fast_row(a.rot + 9 * (size_t)f + 3 * threadIdx.x, a.row_limit2) ? 1u : FLAG_GENERAL;
             for (uint64_t i = b + threadIdx.x; i < e; i += nthr) m = max(m, fast_count(a.walk.photons[i]));
@@ -1335,8 +1335,8 @@ __global__ void ac1d_uw_finish_kernel(const unsigned long long *__restrict__ dev
 
 typedef void (*PairKernel)(SparseArgs);
 
-// dynamic shared memory at most: the boxes of an SM's CTAs, and the histograms of an AC1D CTA
-constexpr size_t PAIR_BOX_BYTES = 184u << 10, AC1D_HIST_BYTES = 216u << 10;
+constexpr size_t pair_box_bytes(int r) { return sizeof(uint32_t) * (r + 1) * (2 * r + 1) * (2 * r + 1); }
+constexpr size_t AC1D_HIST_BYTES = 216u << 10;  // of an AC1D CTA's histograms at most
 
 static PairKernel pick_kernel(int dmap, int i1, int i2)
 {
@@ -1350,7 +1350,7 @@ iac_status pair_kernel_limits()
     const PairKernel pair[] = {sparse_pairs_kernel<0, 0, 0>, sparse_pairs_kernel<0, 0, 1>, sparse_pairs_kernel<1, 0, 0>,
                                sparse_pairs_kernel<1, 0, 1>, sparse_pairs_kernel<1, 1, 0>, sparse_pairs_kernel<1, 1, 1>};
     for (PairKernel k : pair)
-        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_BOX_BYTES));
+        IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_box_bytes(BOX_R_MAX)));
     for (auto k : {ac1d_sparse_kernel<0>, ac1d_sparse_kernel<1>})
         IAC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AC1D_HIST_BYTES));
     return IAC_OK;
@@ -1415,23 +1415,14 @@ static iac_status check_params(const iac_sparse_params *p)
     return IAC_OK;
 }
 
-// The launch shape of a tuning setting: the threads that block_threads x
-// ctas_per_sm asks for on an SM, in as few CTAs as hold them, since the warps
-// of one CTA share one box and a larger box keeps more adds out of L2.
-struct PairShape {
-    int ctas, threads;  // per SM, per CTA
-    int box_max;
-};
-static PairShape pair_shape(const iac_sparse_tuning &tun, int max_threads, int C)
+// Threads of a CTA: block_threads x ctas_per_sm of the tuning setting, up to
+// max_threads, which take all of an SM's registers.  The warps of a CTA share one box,
+// and a larger box keeps more adds out of L2.  Settings of 2 048 and 4 096 threads an
+// SM, 200 frames: 88 and 158 us as two and four CTAs, which wait for one another, 33
+// as one.
+static int pair_cta_threads(const iac_sparse_tuning &tun, int max_threads)
 {
-    const int total = (int)(tun.block_threads * tun.ctas_per_sm);
-    PairShape s;
-    s.ctas = (total + max_threads - 1) / max_threads;
-    s.threads = std::max(32, std::min(max_threads, (total / s.ctas + 31) / 32 * 32));
-    const int budget = (int)PAIR_BOX_BYTES / s.ctas;
-    s.box_max = std::min(BOX_R_MAX, C);
-    while (s.box_max >= 0 && 4 * (s.box_max + 1) * (2 * s.box_max + 1) * (2 * s.box_max + 1) > budget) s.box_max--;
-    return s;
+    return std::max(32, std::min(max_threads, (int)(tun.block_threads * tun.ctas_per_sm) / 32 * 32));
 }
 
 // Plan of one batch: planner header, table of frame starts
@@ -1452,8 +1443,13 @@ static iac_status launch_pair_batch(iac_ctx *ctx, const float *d_photons, const 
     const iac_sparse_tuning tun = effective_tuning(ctx, p->shape.size_ab);
     const int i1 = p->double_map ? p->interp_first : 0;
     const int C = ((int)p->shape.size_ab - 1) / 2;
-    const PairShape sh = pair_shape(tun, pair_threads(p->double_map, i1, p->interp_second), C);
-    const int grid = ctx->sm_count * sh.ctas;
+    const int threads = pair_cta_threads(tun, pair_threads(p->double_map, i1, p->interp_second));
+    // one CTA an SM.  A first-level linear pair is 8 or 64 pairs' work: two CTAs an SM, one
+    // after the other, and the smaller box that two had, even out the ends and leave the
+    // walk its L1 (3 000 frames nearest on the second level 1342 us; one CTA 1395, with
+    // R = 22 1464; 200 frames 142, 156 and 156)
+    const bool heavy = p->double_map && i1;
+    const int grid = ctx->sm_count * (heavy ? 2 : 1);
     const bool direct = nframes <= PAIR_DIRECT;
     SparseArgs a{};
     a.walk.photons = reinterpret_cast<const float4 *>(d_photons);
@@ -1481,7 +1477,7 @@ static iac_status launch_pair_batch(iac_ctx *ctx, const float *d_photons, const 
     a.check_here = direct ? 1 : 0;
     a.flags = q.flags;
     a.cache_hints = tun.cache_hints == 1 ? 1 : 0;
-    a.box_max = sh.box_max;
+    a.box_max = std::min(heavy ? BOX_R_HEAVY : BOX_R_MAX, C);
     // |x| <= |row| (MaxQ Voxel_per_dq + the first level's rounding) < C + 1/2, with a margin for FP32
     const double reach = ((double)p->shape.max_q * p->shape.voxel_per_dq + 0.8661) * 1.00001;
     const double limit = ((double)C + 0.49) / reach;
@@ -1492,14 +1488,14 @@ static iac_status launch_pair_batch(iac_ctx *ctx, const float *d_photons, const 
                                                   2u * (unsigned)ctx->sm_count);
         const unsigned ctas = PLAN_CTAS + (check + PLAN_CTAS - 1) / PLAN_CTAS * PLAN_CTAS;
         sparse_plan_kernel<<<ctas, PLAN_THREADS, 0, s>>>(d_off, nframes, a.walk.steps_max,
-                                                         (uint32_t)(grid * sh.threads / 32), q.cost_off, q.head,
+                                                         (uint32_t)(grid * threads / 32), q.cost_off, q.head,
                                                          a.walk.photons, d_rot9, a.row_limit2, q.flags);
         IAC_LAUNCHED(ctx);
         IAC_CUDA(cudaGetLastError());
     }
-    const size_t box_bytes = sizeof(uint32_t) * (size_t)(sh.box_max + 1) * (2 * sh.box_max + 1) * (2 * sh.box_max + 1);
+    const size_t box_bytes = pair_box_bytes(a.box_max);
     const PairKernel k = pick_kernel(p->double_map, p->interp_first, p->interp_second);
-    k<<<grid, sh.threads, box_bytes, s>>>(a);
+    k<<<grid, threads, box_bytes, s>>>(a);
     IAC_LAUNCHED(ctx);
     IAC_CUDA(cudaGetLastError());
     return IAC_OK;
