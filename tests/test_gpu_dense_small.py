@@ -142,3 +142,39 @@ def test_cq_maxq_that_bounds_nothing(ctx, oracle_lib, rng, interp):
         ctx.cq_small(_dev(I), _dev(km), I.size, to_capi_shape(s), interp, 123457.0, out, fast_size=31)
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want)
     ctx.check()
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+@pytest.mark.parametrize("lit", [0.004, 0.05, 0.5, 1.0])
+@pytest.mark.parametrize("sign", ["positive", "some negative", "bright"])
+def test_maps_of_few_lit_pixels(ctx, oracle_lib, rng, interp, lit, sign):
+    """Tiles of which none, one, an odd number, most or all pixels are lit, in both
+    dense kernels: values of every kind, the masked pixels' k far outside."""
+    from incohautocorrelate_b200 import capi
+    o = oracle_lib
+    ny, nx = 37, 44
+    _, km, mq = small_detector(ny, nx, 6e-4)
+    I = rng.uniform(0.05, 1.5, ny * nx).astype(np.float32)
+    I[rng.random(I.size) >= lit] = 0
+    I[-1] = 1.0
+    if sign == "some negative":
+        I[::3] *= -1
+    elif sign == "bright":
+        I[::5] *= 3000
+    k = km.copy().reshape(-1, 3)
+    k[I == 0] = np.float32(1e18)
+    k = np.ascontiguousarray(k.reshape(-1))
+    s = o.small_cq_mesh_shape(mq, 41)
+    want = np.zeros(s.size_ab * s.size_ab * s.size_c, np.uint64)
+    o.lib().iaco_cq_small(o.p(I), o.p(k), I.size, s, interp, 123457.0, 0, I.size, o.p(want))
+    for fast in (0, nx):
+        out = _dev(np.zeros(want.size, np.int64))
+        ctx.cq_small(_dev(I), _dev(k), I.size, to_capi_shape(s), interp, 123457.0, out, fast_size=fast)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=str(fast))
+    for mult in (123457.0, 100000.5):
+        so, sh = o.ac1d_shape(mq, 300), capi.ac1d_shape(mq, 300)
+        want = np.zeros(sh.size, np.uint64)
+        o.lib().iaco_ac1d_cq(o.p(I), o.p(k), I.size, so, interp, mult, 0, I.size, o.p(want))
+        out = _dev(np.zeros(want.size, np.int64))
+        ctx.ac1d_cq(_dev(I), _dev(k), I.size, sh, interp, mult, out)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want, err_msg=str(mult))
