@@ -1088,7 +1088,9 @@ __device__ __forceinline__ void host_route_add(unsigned long long *whole, uint32
             atomicAdd(&frac[bin], (double)v);
         return;
     }
-    if (v == truncf(v) && v < 1.8e19f)
+    if (v >= 8388608.0f && v < 4294967296.0f)  // a whole number of 32 bits
+        shared_add_u64_split(lo, hi, bin, (unsigned long long)__float2uint_rz(v));
+    else if (v == truncf(v) && v < 1.8e19f)
         shared_add_u64_split(lo, hi, bin, (unsigned long long)__float2ull_rz(v));
     else
         atomicAdd(&frac[bin], (double)v);
@@ -1195,15 +1197,15 @@ __global__ void __launch_bounds__(2 * AC1D_THREADS, 1) ac1d_sparse_kernel(const 
                         rare[e] = on[e] && !fast;
                         u[e] = on[e] && fast ? u[e] : 0u;
                     }
+                    if (!__any_sync(0xffffffffu, rare[0] || rare[1])) {
 #pragma unroll
-                    for (int e = 0; e < 2; e++) old[e] = shared_add32(whole + (u[e] ? 4u * bin[e] : 0u), u[e]);
-                    if (old[0] + u[0] < old[0]) shared_add32(whole + 4u * (a.size + bin[0]), 1u);
-                    if (old[1] + u[1] < old[1]) shared_add32(whole + 4u * (a.size + bin[1]), 1u);
-                    if (rare[0] || rare[1]) {
-#pragma unroll 1
+                        for (int e = 0; e < 2; e++) old[e] = shared_add32(whole + (u[e] ? 4u * bin[e] : 0u), u[e]);
+                        if (old[0] + u[0] < old[0]) shared_add32(whole + 4u * (a.size + bin[0]), 1u);
+                        if (old[1] + u[1] < old[1]) shared_add32(whole + 4u * (a.size + bin[1]), 1u);
+                    } else {
+#pragma unroll
                         for (int e = 0; e < 2; e++)
-                            if (e ? rare[1] : rare[0])
-                                host_route_add(h.whole, a.size, a.counters, e ? bin[1] : bin[0], e ? v[1] : v[0]);
+                            if (on[e]) host_route_add(h.whole, a.size, a.counters, bin[e], v[e]);
                     }
                 } else if (host) {
                     uint32_t at[2], bin[2], u[4];
@@ -1229,22 +1231,19 @@ __global__ void __launch_bounds__(2 * AC1D_THREADS, 1) ac1d_sparse_kernel(const 
                         }
                         rare[e] = on[e] && !(ok[0] && ok[1]);
                     }
+                    if (__any_sync(0xffffffffu, (u[0] | u[1] | u[2] | u[3]) != 0u)) {
 #pragma unroll
-                    for (int m = 0; m < 4; m++) c[m] = shared_add32(at[m >> 1] + 4u * (m & 1), u[m]) + u[m] < u[m];
-                    if (c[0] | c[1] | c[2] | c[3]) {
+                        for (int m = 0; m < 4; m++) c[m] = shared_add32(at[m >> 1] + 4u * (m & 1), u[m]) + u[m] < u[m];
+                        if (c[0] | c[1] | c[2] | c[3]) {
 #pragma unroll
-                        for (int m = 0; m < 4; m++)
-                            if (c[m]) shared_add32(at[m >> 1] + 4u * (m & 1) + 4u * a.size, 1u);
+                            for (int m = 0; m < 4; m++)
+                                if (c[m]) shared_add32(at[m >> 1] + 4u * (m & 1) + 4u * a.size, 1u);
+                        }
                     }
                     if (rare[0] || rare[1]) {
-#pragma unroll 1
-                        for (int m = 0; m < 4; m++) {
-                            const bool second = m >= 2;
-                            const uint32_t w = second ? (m & 1 ? u[3] : u[2]) : (m & 1 ? u[1] : u[0]);
-                            if (w == 0 && (second ? on[1] : on[0]))
-                                host_route_add(h.whole, a.size, a.counters, (second ? bin[1] : bin[0]) + (m & 1),
-                                               second ? (m & 1 ? v[3] : v[2]) : (m & 1 ? v[1] : v[0]));
-                        }
+#pragma unroll
+                        for (int m = 0; m < 4; m++)
+                            if (u[m] == 0 && on[m >> 1]) host_route_add(h.whole, a.size, a.counters, bin[m >> 1] + (m & 1), v[m]);
                     }
                 } else {
                     constexpr int N = INTERP ? 2 : 1;  // bins of a pair
