@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(MERGE_THREADS, 1) merge_kernel(const MergeArgs
     const uint32_t nvox = *a.count;
     const uint32_t f0 = blockIdx.y * MERGE_FRAMES;
     const uint32_t nf = min((uint32_t)MERGE_FRAMES, a.nframes - f0);
-    for (uint32_t k = threadIdx.x; k < MERGE_FRAMES * 10; k += MERGE_THREADS) {
+    for (uint32_t k = threadIdx.x; k < (nf + 1) / 2 * 20; k += MERGE_THREADS) {
         const uint32_t f = k / 10, e = k - 10 * f;
         const float r = f < nf ? a.rw[(size_t)f0 * 10 + k] : 0.0f;
         reinterpret_cast<float *>(s_r[f >> 1])[2 * e + (f & 1)] = r;
