@@ -212,12 +212,20 @@ __device__ __forceinline__ float frame_value(float t, bool masked, int m, float 
 // A sum starts with a few such rounds (the binade doubles with the pixel count)
 // and then meets a tie or a new binade every few chunks.  Where the rounds do not
 // get far (the first pixels, a sum that hovers around zero), the adding thread
-// takes more pixels each time, up to the whole chunk.
+// takes more pixels each time, up to the whole chunk: a round costs as much as some
+// 500 pixels of its chain.
 // 300 frames of 1024 x 512 in 0.28 ms (frame_sums_kernel, the chain of adds:
 // 1.84 ms), 0.097 at the copy rate: bound by the latency of a chunk's block sum
-// and by the few ordered scans, with two or three frames per SM.
+// and by the few ordered scans, with two or three frames per SM.  Of zero-mean noise,
+// where the sums hover, 1.87 with the pixels' pass (chains 1.95; 2.22 with pixels taken
+// one run at a time until a round stalls).
 constexpr int SCAN_RUN = 16;
-constexpr int SCAN_PITCH = SCAN_RUN + 1;  // a run per thread, without bank conflicts
+constexpr int SCAN_PITCH = SCAN_RUN + 4;  // a run per thread in 16-byte words, without bank conflicts
+// The first SCAN_ROUNDS rounds of a chunk get far if they pass as many runs as the adding
+// thread takes, further ones if they pass SCAN_FAR; one that does not doubles what the
+// thread takes (further ones: four times as much, SCAN_MORE at least), one that does
+// halves it.
+constexpr int SCAN_ROUNDS = 4, SCAN_MORE = 16, SCAN_FAR = 64, SCAN_DECAY = 2;
 constexpr float SCAN_MAGIC = 12582912.0f;  // 1.5 * 2^23: z + SCAN_MAGIC rounds |z| < 2^22 to an integer
 
 // a run of pixels: its increment of A for an even and an odd A before it
@@ -229,14 +237,33 @@ __device__ __forceinline__ ParityMap then(ParityMap a, ParityMap b)
     return {a.even + ((a.even & 1) ? b.odd : b.even), a.odd + ((a.odd & 1) ? b.even : b.odd)};
 }
 
+// s plus the pixels of `left` runs, one by one, eight loaded ahead of the chain of
+// adds (unrolled, it spills registers of every chunk: 300 frames with a mask 368 -> 571 us)
+static __device__ __forceinline__ float add_runs(const float *own, int left, float s)
+{
+    const float4 *at = reinterpret_cast<const float4 *>(own);
+    float4 a0 = at[0], a1 = at[1];
+#pragma unroll 1
+    for (; left > 0; left--) {
+        const float4 b0 = at[2], b1 = at[3];
+        s = fadd(fadd(fadd(fadd(s, a0.x), a0.y), a0.z), a0.w);
+        s = fadd(fadd(fadd(fadd(s, a1.x), a1.y), a1.z), a1.w);
+        if (left > 1) at += SCAN_PITCH / 4;
+        a0 = at[0], a1 = at[1];
+        s = fadd(fadd(fadd(fadd(s, b0.x), b0.y), b0.z), b0.w);
+        s = fadd(fadd(fadd(fadd(s, b1.x), b1.y), b1.z), b1.w);
+    }
+    return s;
+}
+
 template <bool VEC, int SCAN_THREADS>
 __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
     frame_scan_kernel(const float *__restrict__ frames, uint64_t npix, const int *__restrict__ mask, float thr,
                       float step, const int *__restrict__ only, float *__restrict__ mean, float *__restrict__ count)
 {
     constexpr int WARPS = SCAN_THREADS / 32, SCAN_PIX = SCAN_THREADS * SCAN_RUN;
-    __shared__ float s_x[SCAN_THREADS * SCAN_PITCH];
-    __shared__ int s_red[2][WARPS][3];  // by chunk parity: increments, their sizes, needs the scan
+    __shared__ __align__(16) float s_x[SCAN_THREADS * SCAN_PITCH];
+    __shared__ int4 s_red[2][WARPS];  // by chunk parity: increments, their sizes, needs the scan
     __shared__ ParityMap s_map[WARPS];
     __shared__ int s_first[WARPS];
     __shared__ float s_acc;
@@ -275,7 +302,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
         scale = __uint_as_float(((uint32_t)(277 - e) << 23) | (b & 0x80000000u));  // 2^(150 - e)
         return true;
     };
-    int runs = 1;  // that the adding thread takes; twice as many after a round that did not get as far
+    int runs = 1;  // that the adding thread takes
     load(0);
     for (uint64_t p0 = 0, c = 0; p0 < npix; p0 += SCAN_PIX, c++) {
         float x[SCAN_RUN];
@@ -316,12 +343,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
             for (int e = 0; e < SCAN_RUN; e++) some |= !(x[e] == 0.0f);
             scan = __any_sync(0xffffffffu, some);
         }
-        int (*red)[3] = s_red[c & 1];
-        if (lane == 0) red[warp][0] = inc, red[warp][1] = size, red[warp][2] = scan;
+        if (lane == 0) s_red[c & 1][warp] = make_int4(inc, size, scan, 0);
         __syncthreads();
-        int ti = 0, ts = 0, need = 0;
-#pragma unroll
-        for (int w = 0; w < WARPS; w++) ti += red[w][0], ts += red[w][1], need |= red[w][2];
+        const int4 of_warp = lane < WARPS ? s_red[c & 1][lane] : make_int4(0, 0, 0, 0);
+        const int ti = __reduce_add_sync(0xffffffffu, of_warp.x), ts = __reduce_add_sync(0xffffffffu, of_warp.y),
+                  need = __any_sync(0xffffffffu, of_warp.z);
         const int up = (ts + ti) >> 1, down = (ts - ti) >> 1;
         if (!need && (!ok || (A + up < (1 << 24) && A - down > (1 << 23)))) {
             if (ok) acc = fmul((float)(A + ti), __uint_as_float((__float_as_uint(acc) & 0x80000000u) |
@@ -330,8 +356,15 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
         }
         // ordered scan; s_x is free: every thread has passed the barrier above
 #pragma unroll
-        for (int e = 0; e < SCAN_RUN; e++) s_x[slot(e) / SCAN_RUN * SCAN_PITCH + slot(e) % SCAN_RUN] = x[e];
+        for (int e = 0; e < SCAN_RUN; e += VEC ? 4 : 1) {
+            float *to = s_x + slot(e) / SCAN_RUN * SCAN_PITCH + slot(e) % SCAN_RUN;
+            if (VEC)
+                *reinterpret_cast<float4 *>(to) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+            else
+                *to = x[e];
+        }
         const float *own = s_x + tid * SCAN_PITCH;
+        int rounds = 0;
         for (int t0 = 0; t0 < SCAN_THREADS;) {
             __syncthreads();  // s_x written, the previous round's results read
             const bool good = binade(scale, A);
@@ -341,9 +374,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
                 float sum = 0.0f, size = 0.0f, ties = 0.0f;
                 bool some = false;
                 const float by = good ? scale : 1.0f;
+                float4 q;
 #pragma unroll
                 for (int e = 0; e < SCAN_RUN; e++) {
-                    const float z = fmul(own[e], by), r = fsub(fadd(z, SCAN_MAGIC), SCAN_MAGIC);
+                    if (e % 4 == 0) q = *reinterpret_cast<const float4 *>(own + e);
+                    const float z = fmul(e % 4 == 0 ? q.x : e % 4 == 1 ? q.y : e % 4 == 2 ? q.z : q.w, by), r = fsub(fadd(z, SCAN_MAGIC), SCAN_MAGIC);
                     ties = fabsf(fsub(z, r)) == 0.5f ? fadd(ties, 1.0f) : ties;
                     some |= !(z == 0.0f);
                     sum = fadd(sum, r);
@@ -380,6 +415,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
             if (lane == 0) before = {0, 0};
             __syncthreads();
             ParityMap ahead{0, 0}, all{0, 0};
+#pragma unroll 2
             for (int w = 0; w < WARPS; w++) {
                 if (w == warp) ahead = all;
                 all = then(all, s_map[w]);
@@ -399,22 +435,14 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1024 / SCAN_THREADS)
                 if (good) acc = fmul((float)(A + ((A & 1) ? all.odd : all.even)), unit);
                 break;
             }
-            if (good) runs = first - t0 < runs ? min(2 * runs, SCAN_THREADS) : 1;
             const int behind = min(SCAN_THREADS, first + (good ? runs : 32));
+            if (good) {
+                const bool far = first - t0 >= (rounds < SCAN_ROUNDS ? runs : SCAN_FAR);
+                runs = far ? max(1, runs / SCAN_DECAY) : min(rounds < SCAN_ROUNDS ? 2 * runs : max(SCAN_MORE, 4 * runs), SCAN_THREADS);
+                rounds++;
+            }
             if (tid == first) {
-                float s = good ? fmul((float)start, unit) : acc;
-                float v[SCAN_RUN], next[SCAN_RUN];
-#pragma unroll
-                for (int e = 0; e < SCAN_RUN; e++) next[e] = own[e];
-                for (const float *run = own; run != s_x + behind * SCAN_PITCH;) {
-                    run += SCAN_PITCH;
-                    const float *ahead_of = run != s_x + behind * SCAN_PITCH ? run : own;
-#pragma unroll
-                    for (int e = 0; e < SCAN_RUN; e++) v[e] = next[e], next[e] = ahead_of[e];
-#pragma unroll
-                    for (int e = 0; e < SCAN_RUN; e++) s = fadd(s, v[e]);
-                }
-                s_acc = s;
+                s_acc = add_runs(own, behind - first, good ? fmul((float)start, unit) : acc);
             }
             __syncthreads();
             acc = s_acc;
@@ -632,16 +660,17 @@ iac_status launch_sums_fpc(int sms, const float *frames, uint64_t npix, uint32_t
 // with some ten rounds of their ordered scan: frames of 100 x 100, 100 of them
 // 41 us (chains 56) but 1 000 of them 147 (121); frames of 200 x 200, 600 of them
 // 171 (225); one frame of 300 x 300 58 (325).  Frames without a signal, whose sums
-// hover around zero, are added nearly pixel by pixel either way (300 of 512 x 1024:
-// 2.1 ms, chains 1.9), so batches of many frames per SM, which the chains take 8 and
-// more to a CTA, stay with them (2 000 of 300 x 300: 0.62 ms, chains 0.74, but
-// without a signal 1.3 and 0.74).
+// hover around zero, are added nearly pixel by pixel either way (zero-mean noise, 300
+// frames of 512 x 1024: 1.87 ms, chains 1.95; of 300 x 300 375 us and 363, 1 184 of them
+// 660 and 599, with a signal 298 and 599), so batches of many frames per SM, which the
+// chains take 8 and more to a CTA, stay with them where a signal gains little (1 184 of
+// 128 x 128: 185 us either way, noise 240 and 184).
 iac_status launch_frame_sums(iac_ctx *ctx, const float *frames, uint64_t npix, uint32_t nframes, const int *mask,
                              float thr, float step, const int *only, float *mean, float *count, cudaStream_t s)
 {
     const bool vec = npix % 4 == 0 && ((uintptr_t)frames & 15) == 0 && ((uintptr_t)mask & 15) == 0;
     const int sms = ctx->sm_count;
-    const bool scan = (npix >= 16384 && nframes <= 8u * sms) || (npix >= 8192 && nframes <= 2u * sms);
+    const bool scan = nframes <= (npix >= 32768 ? 8u : npix >= 16384 ? 5u : npix >= 8192 ? 2u : 0u) * sms;
     if (scan) {
         // smaller CTAs once every SM has its two frames (2 000 frames of 300 x 300: 509 us
         // with 128 threads, 608 with 256; 250 of 512 x 1024: 341 and 316)
