@@ -341,14 +341,25 @@ struct Share {
     uint32_t chunk;  // cost a warp takes at a time
     uint32_t most;
 };
+// A chunk: about four a warp at least, whole units, few enough frame searches, and so
+// many of the cost that its 32-bit counter holds them.
+__host__ __device__ constexpr uint32_t chunk_cost(unsigned long long cost, uint32_t ctas, uint32_t threads, uint32_t steps)
+{
+    unsigned long long c = cost / ctas / (threads / 8);
+    c = c > 128 ? 128 : c;
+    c = c < steps + PAIR_UNIT_COST ? steps + PAIR_UNIT_COST : c;
+    return (uint32_t)(c < (cost >> 31) ? cost >> 31 : c);
+}
+static_assert(chunk_cost(1ull << 16, 148, 1024, 2) == 5 && chunk_cost(1ull << 30, 148, 1024, 32) == 128 &&
+                  chunk_cost(1ull << 40, 148, 1024, 32) == 512 && (1ull << 50) / chunk_cost(1ull << 50, 1, 32, 32) <= 1ull << 31,
+              "the chunks of a batch fit the counter");
 __device__ __forceinline__ Share cta_share(const PlanHeader &h, bool whole)
 {
     Share s;
     s.x0 = whole ? 0ull : h.cost * blockIdx.x / gridDim.x;
     s.x1 = whole ? h.cost : h.cost * (blockIdx.x + 1) / gridDim.x;
-    // about four chunks a warp at least, whole units, and few enough frame searches
     const unsigned long long part = h.cost / gridDim.x;
-    s.chunk = (uint32_t)max((unsigned long long)(h.steps + PAIR_UNIT_COST), min(128ull, part / (blockDim.x / 8)));
+    s.chunk = chunk_cost(h.cost, gridDim.x, blockDim.x, h.steps);
     s.most = (uint32_t)min(0x7fffffffull, 2 * part / s.chunk + 64);
     return s;
 }
