@@ -474,7 +474,7 @@ __device__ __forceinline__ void cq_pairs_win2(const DenseArgs &a, const Window &
     const int words = D01 * w.dim[2];
     const int base = (a.cab - w.lo[0]) + D0 * (a.cab - w.lo[1]) + D01 * (a.cc - w.lo[2]);
     const float2 vp2 = make_float2(a.vpdq, a.vpdq), K0 = make_float2(k0, k0), K1 = make_float2(k1, k1),
-                 K2 = make_float2(k2, k2), IA = make_float2(Ia, Ia);
+                 K2 = make_float2(k2, k2), IA = make_float2(Ia, Ia), nz = make_float2(a.neg_zero, a.neg_zero);
     int cur = 0;  // pending run: window index cur, value acc (0 before the first pair)
     unsigned long long acc = 0;
     auto step = [&](int jp, bool lo_on) {
@@ -487,9 +487,9 @@ __device__ __forceinline__ void cq_pairs_win2(const DenseArgs &a, const Window &
             ok0 = ok0 && !(fadd(fadd(fmul(qx.x, qx.x), fmul(qy.x, qy.x)), fmul(qz.x, qz.x)) > a.maxq2);
             ok1 = ok1 && !(fadd(fadd(fmul(qx.y, qx.y), fmul(qy.y, qy.y)), fmul(qz.y, qz.y)) > a.maxq2);
         }
-        qx = f2mul(qx, vp2);
-        qy = f2mul(qy, vp2);
-        qz = f2mul(qz, vp2);
+        qx = f2fma(qx, vp2, nz);  // an add follows
+        qy = f2fma(qy, vp2, nz);
+        qz = f2fma(qz, vp2, nz);
         const int2 f = f2round_half_away(KA == 0 ? qx : KA == 1 ? qy : qz);
         const int2 m = f2round_half_away(KB == 0 ? qx : KB == 1 ? qy : qz);
         const int2 sz = f2round_half_away(KC == 0 ? qx : KC == 1 ? qy : qz);
@@ -513,7 +513,7 @@ __device__ __forceinline__ void cq_pairs_win2(const DenseArgs &a, const Window &
 // runs, so neither word overflows and no add has to return anything.  Pixels of
 // intensity 0 (masked, or absent from a ragged tile) are not staged; an odd rest is
 // filled up at a corner of the tile's box, so that every pair lands in the window.
-// 1024 x 512 map with 5 % masked, 199-edge mesh, nearest: 214.9 -> 139.4 ms (147.4 with
+// 1024 x 512 map with 5 % masked, 199-edge mesh, nearest: 214.9 -> 141.8 ms (147.4 with
 // the masked pixels staged); linear at 244 x 250, 127-edge mesh: 17.6 -> 7.5 ms (8.4).
 // Larger products keep the 64-bit paths above.
 // ---------------------------------------------------------------------------
@@ -606,10 +606,10 @@ __device__ __forceinline__ void cq_pairs_small(const DenseArgs &a, const Window 
             ok0 = ok0 && !(s.x > a.maxq2);  // a MaxQ that is no number bounds nothing
             ok1 = !(s.y > a.maxq2);
         }
-        const float2 vp = dup(a.vpdq);
-        qx = f2mul(qx, vp);
-        qy = f2mul(qy, vp);
-        qz = f2mul(qz, vp);
+        const float2 vp = dup(a.vpdq), zero = dup(a.neg_zero);  // products that an add follows
+        qx = f2fma(qx, vp, zero);
+        qy = f2fma(qy, vp, zero);
+        qz = f2fma(qz, vp, zero);
         const int2 f = f2round_half_away(KA == 0 ? qx : KA == 1 ? qy : qz);
         const int2 m = f2round_half_away(KB == 0 ? qx : KB == 1 ? qy : qz);
         const int2 sz = f2round_half_away(KC == 0 ? qx : KC == 1 ? qy : qz);
