@@ -2041,14 +2041,25 @@ static void zcol_work_split(TmaGeom &g, long long ncols, int D, long long grid)
 // by that stage or a later one (its stage j - niss waited for the drains of
 // stage j - niss - nb, which follow every earlier stage's MMAs: S >= niss + nb).
 // Otherwise two loads that land out of order are enough to break the ring.
-static int ring_stages(int fit, int niss, int nb)
+static constexpr int ring_stages(int fit, int niss, int nb)
 {
     return fit >= niss + nb ? fit : fit - fit % niss;
 }
+static constexpr bool ring_stages_hold()
+{
+    for (int niss = 2; niss <= 3; niss++)
+        for (int nb = 3; nb <= 5; nb++)
+            for (int fit = niss; fit <= 8; fit++) {
+                const int S = ring_stages(fit, niss, nb);
+                if (S < niss || S > fit || (S % niss != 0 && S < niss + nb)) return false;
+            }
+    return true;
+}
+static_assert(ring_stages_hold(), "stages a multiple of the issuers, or as many as issuers and regions");
 
 // the concatenated-dz z-column convolution (conv_zcat_kernel) when its
-// weights stay resident and 4+ stages fit; false leaves the layer to the
-// others.  IAC_DENOISE_ZCAT=0 in the environment turns it off (for comparing
+// weights stay resident and a ring of two stages or more fits; false leaves the
+// layer to the others.  IAC_DENOISE_ZCAT=0 in the environment turns it off (for comparing
 // the kernels).
 template <int CIN, int COUT>
 static bool launch_zcat(const ConvArgs &a, const TmaGeom &g0, uint32_t budget, cudaStream_t s, cudaError_t &err)

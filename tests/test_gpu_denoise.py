@@ -391,3 +391,29 @@ def test_gradient_buffer_feeds_the_optimizer(ctx, rng):
     finally:
         dn.close()
 
+
+
+@pytest.mark.parametrize("dims", [(1, 128, 128, 128), (2, 96, 96, 96), (1, 32, 48, 64)])
+def test_back_to_back_forwards(ctx, dims):
+    """Whole-mesh forwards one behind the other, whose convolutions run on short rings
+    of stages shared by several issuers: every result is the first one's."""
+    import torch
+    from incohautocorrelate_b200 import capi
+    dn = capi.Denoiser(ctx, *dims, backend=capi.TCGEN05)
+    try:
+        dn.init_params(seed=5)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        x = torch.rand(dims, generator=g, device="cuda")
+        want = torch.zeros_like(x)
+        dn.forward(x, *dims, want)
+        torch.cuda.synchronize()
+        outs = [torch.zeros_like(x) for _ in range(4)]
+        for k in range(200):
+            dn.forward(x, *dims, outs[k % 4])
+        torch.cuda.synchronize()
+        assert ctx.check() == 0
+        assert float(want.abs().sum()) > 0
+        for o in outs:
+            assert torch.equal(o, want)
+    finally:
+        dn.close()
