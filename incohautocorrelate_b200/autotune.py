@@ -25,9 +25,11 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 TABLE = os.path.join(HERE, "tuning", "sparse_tuning.tsv")
 
-GRID = dict(tile_pairs=[2048, 4096, 8192, 16384, 32768],
-            block_threads=[128, 256],
-            ctas_per_sm=[4, 6, 8, 12, 16],
+# settings that differ in the launch: a unit of the walk holds up to 1 024 pairs, and
+# block_threads x ctas_per_sm threads run on an SM, 1 024 at most
+GRID = dict(tile_pairs=[128, 256, 512, 1024],
+            block_threads=[256],
+            ctas_per_sm=[2, 3, 4],
             cache_hints=[2, 1])
 
 
