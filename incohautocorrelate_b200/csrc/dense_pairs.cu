@@ -890,7 +890,7 @@ __device__ __forceinline__ uint32_t wrap_bin(uint32_t b, uint32_t n)
 // cq_pairs_small) and no negative ones, below 2^24 into the split counters; else any,
 // 64 bits each (200 x 220, intensities past the limit, nearest 2.23 -> 1.68 ms, linear
 // 2.83 -> 2.17; some negative 2.45 -> 1.94 and 2.70 -> 1.96).  CHECK: as cq_pairs.
-// 512^2 map with 5 % masked, linear, 88.4 -> 51.8 ms (issue 87 %, conversion unit 40 %);
+// 512^2 map with 5 % masked, linear, 88.4 -> 51.8 ms (issue 88 %, conversion unit 42 %);
 // nearest 78.1 -> 35.8 ms.
 template <int INTERP, bool CHECK, bool SMALL>
 __device__ __forceinline__ void ac1d_pairs(const DenseArgs &a, uint32_t hist, const float4 *sp, int j0, int n,

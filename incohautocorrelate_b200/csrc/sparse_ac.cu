@@ -864,8 +864,8 @@ constexpr int pair_threads(int dmap, int i1, int i2) { return dmap && i1 ? 512 :
 // mesh once, at the end.  Bound by the L2 request rate of the adds outside the
 // box and by issue slots, about evenly: 89 instructions per 32 pairs (164 with
 // a thread per pair, its two loads and its index arithmetic), 100 000 frames
-// 4.2 ms (5.8 with a work queue, a barrier per frame and R = 9), one event of
-// 164 photons 8 us (three launches, 36 us), linear second level on 3.6e7 pairs
+// 4.3 ms (5.8 with a work queue, a barrier per frame and R = 9), one event of
+// 164 photons 10 us (three launches, 36 us), linear second level on 3.6e7 pairs
 // of a 129^3 mesh 0.67 ms (1.5).
 template <int DMAP, int I1, int I2>
 __global__ void __launch_bounds__(pair_threads(DMAP, I1, I2), 1) sparse_pairs_kernel(SparseArgs a)
@@ -1049,8 +1049,8 @@ __global__ void sparse_fold_kernel(const unsigned long long *__restrict__ half, 
 // photons i and step through partners two at a time, the squared distances in
 // f32x2, |q| / dq by the two-word reciprocal; the order of a pair's photons
 // changes neither |q| nor the value.  A unit belongs to one frame, so the route
-// branch is uniform across the warp.  Issue-bound (80 %, 110 instructions a pair):
-// 20 000 frames (2.2e8 pairs, 2048 bins) 1578 -> 910 us linear, 979 -> 590 nearest;
+// branch is uniform across the warp.  Issue-bound (84 %, 117 instructions a pair):
+// 20 000 frames (2.2e8 pairs, 2048 bins) 1578 -> 884 us linear, 979 -> 590 nearest;
 // with double adds the linear walk took 1100.  Device route, 2 000 frames of 230
 // photons, 950 bins: 455 -> 288 us linear, 347 -> 239 nearest.
 // ---------------------------------------------------------------------------
@@ -1082,7 +1082,7 @@ struct AC1DArgs {
 };
 
 // shared-memory histograms of one CTA: 64-bit counters as split 32-bit words
-// (shared_add_u64_split), host-route fractions in units of 2^-32 or as doubles
+// (shared_add_u64_split), host-route fractions in units of fix_top 2^-23 or as doubles
 struct AC1DHist {
     uint32_t *dev_lo, *dev_hi;  // vecsize words each
     unsigned long long *whole;  // size split words, then size doubles
@@ -1129,8 +1129,9 @@ __device__ __forceinline__ void device_route_add(const AC1DArgs &b, const AC1DHi
     if (w) shared_add_u64_split(h.dev_lo, h.dev_hi, wrap_bin(bin, b.vecsize), 2ull * w);
 }
 
-// 20 000 frames, linear, by threads x CTAs per SM: 512 x 2 857 us, 512 x 3 823, 768 x 2
-// 817, 1024 x 1 855; 200 frames 39, 57, 47 and 52: a short batch pays for each CTA.
+// 20 000 frames, linear, by threads x CTAs per SM, before the device route's walk took
+// registers of it: 512 x 2 857 us (884 now), 512 x 3 823, 768 x 2 817, 1024 x 1 855; 200
+// frames 39, 57, 47 and 52: a short batch pays for each CTA.
 constexpr int AC1D_THREADS = 512, AC1D_PER_SM = 2;
 // batches planned by the CTAs themselves: 1000 frames 79 us, with the planner's launch 87
 constexpr uint32_t AC1D_DIRECT = 1024;
